@@ -514,9 +514,9 @@ EMC_API emc_status emc_centred_to_half(const float* d_in, int nx, int ny, int nz
  * :16-30) is sorted on column 1 and cast to single; each particle's defocus is offset by the
  * height of its position along every tilt's beam; the volumes come from emc_sf3d (full grid, CTF
  * squared) and are shifted by -(min - 1e-4).  xyz: [count][3]; recon_geometry: the 2 x 3
- * reconGeometry, row-major (size, then shift); d_out: [count][size^3].  All particles' tilt images
- * are made by one launch per chunk of particles (under 1 GiB of images) and accumulated by a
- * second; the call synchronises the stream once. */
+ * reconGeometry, row-major (size, then shift); d_out: [count][size^3].  The tilt
+ * images are made by one launch per chunk of particles (about 48 MiB of images) and accumulated by
+ * a second; the call synchronises the stream once. */
 EMC_API emc_status emc_sf3d_particles(const unsigned size[3], double sampling, const double* tlt, int rows,
                                       int cols, const double* xyz, const double recon_geometry[6], int count,
                                       float* d_out, void* stream);

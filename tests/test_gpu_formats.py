@@ -123,3 +123,19 @@ def test_sf3d_weight_as_the_search_wedge(built_lib, cuda):
     cc_o, pk_o = O.search(ref, P, mats, radius=6, **kw)
     check_cc_and_peaks(cc, pk, cc_o, pk_o, lambda o: O.xcf_translational(ref, P, mats[o], **kw)[2], "sf3d wedge")
     check_best(best[0][1], cc_o, what="sf3d wedge")
+
+
+@pytest.mark.parametrize("size,tilts,count", [((8, 8, 8), 1, 1), ((33, 40, 20), 33, 5), ((24, 65, 31), 130, 2),
+                                              ((64, 31, 9), 41, 9)])
+def test_sf3d_particles_sizes(built_lib, cuda, size, tilts, count):
+    """Odd and unequal edges, one tilt, more tilts than one list holds, volume groups with a remainder;
+    same tolerance as the cubic case."""
+    from emclarity_b200 import api
+    rng = np.random.default_rng(tilts)
+    t = _tilt_table(rng, tilts)
+    rg = np.array([[512, 512, 256], [0.0, 1.0, -2.0]])
+    xyz = rng.uniform(1, [512, 512, 256], (count, 3))
+    got = api.sf3d_particles(size, 2.0, t, xyz, rg).cpu().numpy()
+    ref = O.sf3d_particles_np(size, 2.0, t, xyz, rg)
+    for g, r in zip(got, ref):
+        assert np.abs(g - r).max() <= 2e-4 * np.abs(r).max(), np.abs(g - r).max()
