@@ -75,3 +75,29 @@ def test_peak_loop_stops_at_threshold_and_tries(built_lib, cuda):
     got_t = api.tsearch_peaks(torch.from_numpy(mag).cuda(), torch.from_numpy(ang).cuda(), removal, rm, al,
                               max_peaks=1000, max_tries=5)
     assert len(got_t) <= 5
+
+
+@pytest.mark.parametrize("shape,size", [((40, 70, 63), 2), ((33, 64, 65), 7), ((20, 129, 128), 16), ((60, 62, 200), 40),
+                                        ((50, 66, 130), 96), ((50, 66, 130), 97), ((44, 200, 2048), 16),
+                                        ((9, 1, 30), 2)])
+def test_moving_average_tiles(built_lib, cuda, shape, size):
+    """Tile edges, narrow tiles, the widest tiled feature and the next one, and several slabs (planes of
+    200 x 2048).  Three passes of `size` products each with weights summing to 1: every output is within
+    3 (size + 2) roundings of the largest input."""
+    from emclarity_b200 import api
+    rng = np.random.default_rng(size)
+    v = rng.standard_normal(shape).astype(np.float32)
+    got = api.moving_average(torch.from_numpy(v).cuda(), size).cpu().numpy()
+    ref = O.moving_average_np(v, size)
+    bound = 3 * (size + 2) * 2.0 ** -24
+    assert np.abs(got - ref).max() <= bound * np.abs(v).max()
+    # in place, the same sums for x and x^2: the error of the quotient from those of its parts
+    loc = api.local_normalize(torch.from_numpy(v).cuda(), size).cpu().numpy()
+    x = v.astype(np.float64)
+    a2 = O.moving_average_np(x * x, size)
+    var = a2 - ref * ref
+    ok = var > 0.05
+    e1, e2 = bound * np.abs(x).max(), (bound + 2.0 ** -24) * (x * x).max()
+    tol = (e1 + np.abs(x - ref) * (e2 + 2 * np.abs(ref) * e1 + e1 * e1) / (2 * var.clip(0.05))) / np.sqrt(var.clip(0.05))
+    want = (x - ref) / np.sqrt(var.clip(0.05))
+    assert ok.any() and np.all(np.abs(loc - want)[ok] <= (2 * tol + 8 * 2.0 ** -24 * np.abs(want))[ok])
