@@ -108,6 +108,23 @@ __device__ __forceinline__ unsigned long long ffma2(unsigned long long a, unsign
   return d;
 }
 
+__device__ __forceinline__ unsigned long long fmul2(unsigned long long a, unsigned long long b) {
+  unsigned long long d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ unsigned long long fadd2(unsigned long long a, unsigned long long b) {
+  unsigned long long d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+// rounds towards minus infinity
+__device__ __forceinline__ unsigned long long fadd2_rd(unsigned long long a, unsigned long long b) {
+  unsigned long long d;
+  asm("add.rm.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+
 // Bulk global -> shared copies through the tensor-memory-access unit (cp.async.bulk, this CTA's
 // own shared memory, no multicast), completed on a shared-memory mbarrier by transaction count.
 // Source and destination 16-byte aligned, size a multiple of 16.

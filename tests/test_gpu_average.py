@@ -110,3 +110,22 @@ def test_empty_half_set_is_nan_and_bad_arguments(built_lib, cuda):
     with pytest.raises(EmcError):
         api.Average(torch.zeros(8, 8, 8, device="cuda"))  # no voxel above the threshold
     avg.close()
+
+
+@pytest.mark.parametrize("n,nw", [(33, 17), (34, 9), (16, 16), (50, 48)])
+def test_brick_edges_and_wide_matrices(built_lib, cuda, n, nw):
+    """Edges that end inside a brick and each copy width (odd, even and multiple-of-four boxes), and
+    matrices that scale by 2.5 (their source box is larger than the staging, so the samples come from
+    global memory) beside rotations; same tolerance as the other boxes."""
+    c = _case(20 + n, n=n, k=4, nw=nw)
+    c["rots"][1] = 2.5 * c["rots"][1]
+    c["shifts"][2] = (40.0 * n, 0.0, 0.0)  # the window of particle 2 lies outside: no finite rms, dropped
+    g, kept = _run_gpu(c)
+    with np.errstate(invalid="ignore", divide="ignore"):
+        o, kept_o = _run_oracle(c)
+    assert list(kept) == list(kept_o) == [True, True, False, True]
+    for h in (1, 2):
+        assert g[h][2] == o[h][2]
+        for k in (0, 1):
+            a, b = g[h][k].cpu().numpy(), o[h][k]
+            assert np.abs(a - b).max() <= 2e-5 * np.abs(b).max(), (h, k)
