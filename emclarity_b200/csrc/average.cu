@@ -121,12 +121,6 @@ constexpr int kBrickXY = 16, kBrickZ = 8;
 constexpr int kBoxYZ = 26, kBoxX = 28;
 constexpr size_t kAvgBoxBytes = sizeof(float) * kBoxX * kBoxYZ * kBoxYZ;
 
-// floor(s) for |s| < 2^22 by a round-down addition that leaves the integer in the low mantissa bits
-// (the conversion instructions run at a quarter of the rate): the bits of r minus kFloorBits are the
-// integer, r - kFloorMagic the same value as a float, exactly.
-constexpr float kFloorMagic = 12582912.f;  // 1.5 2^23
-constexpr unsigned kFloorBits = 0x4b400000u;
-
 // avg_sample_border of two samples (register pairs) from the staged box: same weights, same order, one
 // packed FP32 instruction for both.  Samples outside the volume read staged zeros.  base: offset of
 // the box for the raw mantissa bits of the three floors.

@@ -124,6 +124,27 @@ template <int SIGN> struct Dft<16, SIGN> {
   }
 };
 
+// 12 = 3 x 4, coprime factors: with n = 4 n1 + 3 n2 and k = 4 k1 + 9 k2 (mod 12) the transform is three
+// 4-point and four 3-point transforms without twiddles (Good, 1958).
+template <int SIGN> struct Dft<12, SIGN> {
+  static __host__ __device__ __forceinline__ void run(float2* v) {
+    float2 t[3][4];
+#pragma unroll
+    for (int n1 = 0; n1 < 3; ++n1) {
+#pragma unroll
+      for (int n2 = 0; n2 < 4; ++n2) t[n1][n2] = v[(4 * n1 + 3 * n2) % 12];
+      Dft<4, SIGN>::run(t[n1]);
+    }
+#pragma unroll
+    for (int k2 = 0; k2 < 4; ++k2) {
+      float2 u[3] = {t[0][k2], t[1][k2], t[2][k2]};
+      Dft<3, SIGN>::run(u);
+#pragma unroll
+      for (int k1 = 0; k1 < 3; ++k1) v[(4 * k1 + 9 * k2) % 12] = u[k1];
+    }
+  }
+};
+
 // cos / sin(2 pi j / R) for the odd prime radices 5, 7 and 13 (exact values rounded to float).
 __host__ __device__ constexpr float prime_cos(int R, int j) {
   return R == 5 ? (j == 0 ? 1.f : j == 1 ? 3.09016994374947451e-01f : j == 2 ? -8.09016994374947340e-01f

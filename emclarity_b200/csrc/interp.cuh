@@ -14,6 +14,12 @@ namespace emc {
 // FP32 -> BF16 (round to nearest even) copy of a device array (defined in xform3d.cu).
 emc_status to_bf16(const float* in, __nv_bfloat16* out, long n, cudaStream_t st);
 
+// floor(s) for |s| < 2^22 by a round-down addition that leaves the integer in the low mantissa bits
+// (the conversion instructions run at a quarter of the rate): the bits of r minus kFloorBits are the
+// integer, r - kFloorMagic the same value as a float, exactly.
+constexpr float kFloorMagic = 12582912.f;  // 1.5 2^23
+constexpr unsigned kFloorBits = 0x4b400000u;
+
 template <typename T>
 __device__ __forceinline__ float ldv(const T* p, long i);
 template <>

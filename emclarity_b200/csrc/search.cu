@@ -73,61 +73,35 @@ __global__ void k_search_scatter(const EvalResult* __restrict__ results, long n,
 }
 
 // ------------------------------------------------------------------ per-size dispatch
-// Pass A holds G z-planes per CTA: larger G amortises the per-CTA setup (sampling matrix,
-// twiddles, reductions) over more planes, smaller G raises the number of resident CTAs. The
-// best G depends on the box, the chunk size (wave quantisation over the SMs) and the
-// reference storage type, so it is chosen by timing (tune_planes) rather than fixed.
-constexpr size_t kMaxSmemPerCta = 227 * 1024;
+// Pass A runs g z-planes per CTA one after another: more planes amortise the per-CTA setup
+// (sampling matrix, twiddles, reductions), fewer leave a shorter last wave.  The best g depends on the
+// box, the chunk size and the reference storage type, so it is chosen by timing (tune_planes).
 constexpr int kPlaneOptions[] = {1, 2, 4, 8};
-
-template <int N, int G>
-constexpr bool planes_fit() {
-  return N % G == 0 && SearchCfg<N, G>::SMEM_A <= kMaxSmemPerCta;
-}
-
-template <int N, typename T, int G>
-static emc_status set_attr_fwd() {
-  if constexpr (planes_fit<N, G>())
-    EMC_CUDA(cudaFuncSetAttribute(k_search_fwd_xy<N, T, G>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)SearchCfg<N, G>::SMEM_A));
-  return EMC_OK;
-}
 
 template <int N, typename T>
 static emc_status set_attrs() {
   using C = SearchCfg<N>;
-  EMC_TRY((set_attr_fwd<N, T, 1>()));
-  EMC_TRY((set_attr_fwd<N, T, 2>()));
-  EMC_TRY((set_attr_fwd<N, T, 4>()));
-  EMC_TRY((set_attr_fwd<N, T, 8>()));
+  EMC_CUDA(cudaFuncSetAttribute(k_search_fwd_xy<N, T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)C::SMEM_A));
+  EMC_CUDA(cudaFuncSetAttribute(k_search_fwd_xy<N, T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)C::SMEM_A));
   EMC_CUDA(cudaFuncSetAttribute(k_search_z_mul<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM_B));
   EMC_CUDA(cudaFuncSetAttribute(k_search_inv_peak<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM_C));
   return EMC_OK;
 }
 
-template <int N, typename T, int G>
-static bool launch_fwd_g(const SearchChunkArgs& a, const float2* tw, cudaStream_t st) {
-  if constexpr (planes_fit<N, G>()) {
-    using C = SearchCfg<N, G>;
-    k_search_fwd_xy<N, T, G><<<dim3(N / G, a.n_items), C::NT_A, C::SMEM_A, st>>>(a, tw);
-    return true;
-  }
-  return false;
-}
-
 template <int N, typename T>
-static emc_status launch_fwd(int g, const SearchChunkArgs& a, const float2* tw, cudaStream_t st) {
-  bool ok = false;
-  switch (g) {
-    case 1: ok = launch_fwd_g<N, T, 1>(a, tw, st); break;
-    case 2: ok = launch_fwd_g<N, T, 2>(a, tw, st); break;
-    case 4: ok = launch_fwd_g<N, T, 4>(a, tw, st); break;
-    case 8: ok = launch_fwd_g<N, T, 8>(a, tw, st); break;
-  }
-  if (!ok) {
+static emc_status launch_fwd(int g, const SearchChunkArgs& args, const float2* tw, cudaStream_t st) {
+  using C = SearchCfg<N>;
+  if (!planes_allowed(N, g)) {
     set_error("search: %d planes per CTA not available for box %d", g, N);
     return EMC_E_ARG;
   }
+  SearchChunkArgs a = args;
+  a.planes = g;
+  // (every reference of a handle has its cells)
+  (a.interp == EMC_INTERP_CUBIC ? k_search_fwd_xy<N, T, false> : k_search_fwd_xy<N, T, true>)<<<
+      dim3(N / g, a.n_items), C::NT_A, C::SMEM_A, st>>>(a, tw);
   EMC_LAUNCH_CHECK();
   return EMC_OK;
 }
@@ -143,7 +117,7 @@ static emc_status launch_chunk(int g, const SearchChunkArgs& a, cudaStream_t st,
   if (ev) EMC_CUDA(cudaEventRecord(ev[0], st));
   EMC_TRY((launch_fwd<N, T>(g, a, tw, st)));
   if (ev) EMC_CUDA(cudaEventRecord(ev[1], st));
-  k_search_z_mul<N><<<dim3(C::GRID_BX, (a.n_items + C::EVALS_B - 1) / C::EVALS_B), C::NT_B, C::SMEM_B, st>>>(a, tw);
+  k_search_z_mul<N><<<dim3(N, (a.n_items + C::EVALS_B - 1) / C::EVALS_B), C::NT_B, C::SMEM_B, st>>>(a, tw);
   EMC_LAUNCH_CHECK();
   if (ev) EMC_CUDA(cudaEventRecord(ev[2], st));
   k_search_inv_peak<N><<<dim3(w, a.n_items), C::NT_BC, C::SMEM_C, st>>>(a, tw);
@@ -156,26 +130,8 @@ static bool box_supported(int n) { return n == 64 || n == 96 || n == 128; }
 
 static int box_index(int n) { return n == 64 ? 0 : (n == 96 ? 1 : 2); }
 
-template <int N>
-static bool planes_fit_rt(int g) {
-  switch (g) {
-    case 1: return planes_fit<N, 1>();
-    case 2: return planes_fit<N, 2>();
-    case 4: return planes_fit<N, 4>();
-    case 8: return planes_fit<N, 8>();
-  }
-  return false;
-}
-
-// Whether pass A can run box n with g planes per CTA (g divides n, the slab fits shared memory).
-static bool planes_available(int n, int g) {
-  switch (n) {
-    case 64: return planes_fit_rt<64>(g);
-    case 96: return planes_fit_rt<96>(g);
-    case 128: return planes_fit_rt<128>(g);
-  }
-  return false;
-}
+// Whether pass A runs box n with g planes per CTA.
+static bool planes_available(int n, int g) { return box_supported(n) && planes_allowed(n, g); }
 
 template <typename T>
 static emc_status launch_fwd_any_t(int n, int g, const SearchChunkArgs& a, cudaStream_t st) {
@@ -294,6 +250,8 @@ struct emc_search_s {
     float* wref = nullptr;
     void* cells = nullptr;
     unsigned* mask_rows = nullptr;
+    void* bricks = nullptr;  // pass A's copies of the cells and the mask
+    float* mask_tiles = nullptr;
     int n = 0;
     int dtype = 0;
   };
@@ -471,22 +429,29 @@ emc_status emc_search_add_reference(emc_search_t s, const float* d_ref, int n, c
     EMC_CUDA(cudaMalloc(&r.mask_rows, sizeof(unsigned) * (size_t)n * n));
     emc::k_mask_rows<<<(n * n + 7) / 8, 256, 0, st>>>(r.mask, n, r.mask_rows);
     EMC_LAUNCH_CHECK();
+    EMC_CUDA(cudaMalloc(&r.mask_tiles, nv * sizeof(float)));
+    emc::k_mask_tiles<<<4 * emc::device_sm_count(), 256, 0, st>>>(r.mask, n, r.mask_tiles);
+    EMC_LAUNCH_CHECK();
   }
   if (d_wref) {
     EMC_CUDA(cudaMalloc(&r.wref, nhalf * sizeof(float)));
     EMC_CUDA(cudaMemcpyAsync(r.wref, d_wref, nhalf * sizeof(float), cudaMemcpyDeviceToDevice, st));
   }
   {
-    // trilinear corner cells for the linear interpolation modes
+    // trilinear corner cells for the linear interpolation modes: x fastest (adjoint), bricks (pass A)
     const long nc = (long)(n + 1) * (n + 1) * (n + 1);
     const int blocks = (int)std::min<long>((nc + 255) / 256, 4L * emc::device_sm_count());
-    if (store_dtype == EMC_DTYPE_F32) {
-      EMC_CUDA(cudaMalloc(&r.cells, nc * sizeof(emc::CellT<float>)));
-      emc::k_build_cells<float><<<blocks, 256, 0, st>>>(d_ref, n, (emc::CellT<float>*)r.cells);
-    } else {
-      EMC_CUDA(cudaMalloc(&r.cells, nc * sizeof(emc::CellT<__nv_bfloat16>)));
-      emc::k_build_cells<__nv_bfloat16><<<blocks, 256, 0, st>>>(d_ref, n, (emc::CellT<__nv_bfloat16>*)r.cells);
-    }
+    auto build = [&](auto cell) -> emc_status {
+      using T = decltype(cell);
+      using Cell = emc::CellT<T>;
+      EMC_CUDA(cudaMalloc(&r.cells, nc * sizeof(Cell)));
+      EMC_CUDA(cudaMalloc(&r.bricks, emc::brick_cells(n) * sizeof(Cell)));
+      emc::k_build_cells<T><<<blocks, 256, 0, st>>>(d_ref, n, (Cell*)r.cells);
+      emc::k_build_bricks<T><<<blocks, 256, 0, st>>>(d_ref, n, (Cell*)r.bricks);
+      return EMC_OK;
+    };
+    if (store_dtype == EMC_DTYPE_F32) EMC_TRY(build(float()));
+    else EMC_TRY(build(__nv_bfloat16()));
     EMC_LAUNCH_CHECK();
   }
   EMC_TRY(emc::set_attrs_any(n, store_dtype));
@@ -815,7 +780,7 @@ static emc_status search_run(emc_search_t s, const emc_particle_desc* particles,
     std::vector<emc::DevRef> dr(s->refs.size());
     for (size_t i = 0; i < s->refs.size(); ++i)
       dr[i] = {s->refs[i].data, s->refs[i].mask,  s->refs[i].wref,     s->refs[i].n,
-               s->refs[i].dtype, s->refs[i].cells, s->refs[i].mask_rows};
+               s->refs[i].dtype, s->refs[i].cells, s->refs[i].mask_rows, s->refs[i].bricks, s->refs[i].mask_tiles};
     EMC_TRY(s->d_refs.reserve(dr.size()));
     EMC_CUDA(cudaMemcpy(s->d_refs.p, dr.data(), sizeof(emc::DevRef) * dr.size(), cudaMemcpyHostToDevice));
     s->refs_dirty = false;
@@ -1028,6 +993,8 @@ emc_status emc_search_destroy(emc_search_t s) {
     cudaFree(r.wref);
     cudaFree(r.cells);
     cudaFree(r.mask_rows);
+    cudaFree(r.bricks);
+    cudaFree(r.mask_tiles);
   }
   s->d_refs.release();
   s->d_dmat.release();

@@ -1,17 +1,15 @@
 // search_kernels.cuh -- the three fused passes of one CC evaluation (particle, orientation).
 //
 // Data flow per evaluation e (box n, half width nh = n/2+1, peak radius r, window w = 2r+1):
-//   pass A  (CTA = G z-planes)   gather r = mask .* I(M (p - c - t) + c)  -> smem
-//                                (no weight on the reference: FP64 sums of r and r^2, the
-//                                DC-free energy by Parseval)
-//                                R2C along x (two rows per complex FFT), FFT along y
-//                                -> S1[e][ky][part][z][kx], one padded slab per (ky, column part)
-//                                   in pass B's tile layout                (~n * n * nh c64)
-//   pass B  (CTA = one ky row    slab in by one bulk copy; FFT along z, X = Q .* conj(wref .* R)
-//            or half of one)     .* wdgMask, X(0) = 0, E_R = sum |wref .* R .* wdgMask|^2 when
-//                                either weight is set (formed in registers between the
-//                                transforms, fft_line_fwd_mul_inv), inverse FFT along z, keep the
-//                                w output planes |sz| <= r
+//   pass A  (CTA = z-planes, one gather r = mask .* I(M (p - c - t) + c) into registers
+//            at a time)          (no weight on the reference: sums of r and r^2, the DC-free energy by
+//                                Parseval), R2C along x (two rows per complex FFT), FFT along y,
+//                                in place in one shared-memory plane
+//                                -> S1[e][ky][z][column]                   (~n * n * nh c64)
+//   pass B  (CTA = one ky row)   FFT along z, X = Q .* conj(wref .* R) .* wdgMask, X(0) = 0,
+//                                E_R = sum |wref .* R .* wdgMask|^2 when either weight is set (both
+//                                formed in registers between the transforms), inverse FFT along z,
+//                                keep the w output planes |sz| <= r
 //                                -> S2[e][j][ky][kx], planes in pass C's tile layout  (~w * n * nh c64)
 //   pass C  (CTA = one sz plane) inverse FFT along y, C2R along x for the w rows |sy| <= r,
 //                                normalise by sqrt(E_R E_P), spherical peak mask,
@@ -43,6 +41,8 @@ struct DevRef {
   int dtype;
   const void* cells;   // (n+1)^3 trilinear corner cells (see build_cells) or null
   const unsigned* mask_rows;  // per (z, y) row: lo | hi << 16, the x extent [lo, hi) of mask != 0, or null
+  const void* bricks;         // the corner cells in pass A's bricks (brick_index), or null
+  const float* mask_tiles;    // the mask in pass A's tiles (mask_tile_index), or null
 };
 
 // Trilinear corner cells: cell (i, j, k), i, j, k in [-1, n-1], holds the 8 voxels
@@ -107,56 +107,65 @@ __device__ __forceinline__ long cell_index(int n, float sx, float sy, float sz, 
   return ((long)(z0 + 1) * nc + (y0 + 1)) * nc + (x0 + 1);
 }
 
-// cell_index for the search gather: floor by a round-down conversion, 32-bit index arithmetic,
-// and no clamping -- an invalid sample reads cell 0 and its value is discarded by the caller
-// (`valid` false), so only in-range indices ever reach memory.
-template <int MODE>
-__device__ __forceinline__ unsigned cell_index_gather(int n, float sx, float sy, float sz, float f[3], bool& valid) {
-  valid = MODE == EMC_INTERP_LINEAR_BORDER
-              ? (sx > -1.f && sy > -1.f && sz > -1.f && sx < (float)n && sy < (float)n && sz < (float)n)
-              : (sx >= 0.f && sy >= 0.f && sz >= 0.f && sx <= (float)(n - 1) && sy <= (float)(n - 1) &&
-                 sz <= (float)(n - 1));
-  const int x0 = __float2int_rd(sx), y0 = __float2int_rd(sy), z0 = __float2int_rd(sz);
-  f[0] = sx - (float)x0;
-  f[1] = sy - (float)y0;
-  f[2] = sz - (float)z0;
-  const unsigned nc = (unsigned)n + 1u;
-  const unsigned idx = ((unsigned)(z0 + 1) * nc + (unsigned)(y0 + 1)) * nc + (unsigned)(x0 + 1);
-  return valid ? idx : 0u;
+// Pass A's copies.  A warp of pass A samples patches of 8 (y) x 4 (x) voxels of one plane, and what a
+// warp-wide cell load costs is one L1 wavefront per distinct 128-byte line.  Cells (X, Y, Z), each
+// coordinate one more than the cell's lower corner, are stored as bricks of 2 (y) x 2 (z) cells, y
+// fastest, then x: over random rotations such a patch touches 18.7 lines (FP32; 15.9 with BF16
+// cells), a row of 32 voxels over cells in plain order 26.8.
+__host__ __device__ constexpr unsigned brick_row(int n) { return 4u * (unsigned)((n + 2) / 2); }  // cells per X
+__host__ __device__ constexpr unsigned brick_slab(int n) { return brick_row(n) * (unsigned)(n + 1); }  // per Z pair
+__host__ __device__ constexpr long brick_cells(int n) { return (long)brick_slab(n) * ((n + 2) / 2); }
+__host__ __device__ constexpr unsigned brick_index(int n, unsigned X, unsigned Y, unsigned Z) {
+  return (Z >> 1) * brick_slab(n) + X * brick_row(n) + (Y >> 1) * 4u + (Z & 1u) * 2u + (Y & 1u);
+}
+// The mask in tiles of one patch: a warp reads one 128-byte line.
+__host__ __device__ constexpr int mask_tile_index(int n, int x, int y, int z) {
+  return ((z * (n / 4) + x / 4) * (n / 8) + y / 8) * 32 + (x % 4) * 8 + y % 8;
 }
 
-// Same interpolation order as sample_linear, so both paths give identical results.
-__device__ __forceinline__ float cell_trilinear(const float v[8], const float f[3]) {
-  const float c00 = fmaf(f[0], v[1] - v[0], v[0]), c10 = fmaf(f[0], v[3] - v[2], v[2]);
-  const float c01 = fmaf(f[0], v[5] - v[4], v[4]), c11 = fmaf(f[0], v[7] - v[6], v[6]);
-  const float c0 = fmaf(f[1], c10 - c00, c00), c1 = fmaf(f[1], c11 - c01, c01);
-  return fmaf(f[2], c1 - c0, c0);
+template <typename T>
+__device__ __forceinline__ CellT<T> make_cell(const float* __restrict__ vol, int n, int i, int j, int k) {
+  float v[8];
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    const int x = i + (q & 1), y = j + ((q >> 1) & 1), z = k + ((q >> 2) & 1);
+    v[q] = (x >= 0 && y >= 0 && z >= 0 && x < n && y < n && z < n) ? vol[((long)z * n + y) * n + x] : 0.f;
+  }
+  CellT<T> c;
+  if constexpr (sizeof(T) == 4) {
+    reinterpret_cast<CellT<float>&>(c).lo = make_float4(v[0], v[1], v[2], v[3]);
+    reinterpret_cast<CellT<float>&>(c).hi = make_float4(v[4], v[5], v[6], v[7]);
+  } else {
+    __nv_bfloat162* p = reinterpret_cast<__nv_bfloat162*>(&reinterpret_cast<CellT<__nv_bfloat16>&>(c).v);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) p[q] = __floats2bfloat162_rn(v[2 * q], v[2 * q + 1]);
+  }
+  return c;
 }
 
-// Builds the corner cells of an n^3 FP32 volume, stored as T.
+// Builds the corner cells of an n^3 FP32 volume, stored as T, x fastest.
 template <typename T>
 __global__ void k_build_cells(const float* __restrict__ vol, int n, CellT<T>* __restrict__ cells) {
   const long nc = n + 1;
   const long total = nc * nc * nc;
+  for (long ci = blockIdx.x * (long)blockDim.x + threadIdx.x; ci < total; ci += (long)gridDim.x * blockDim.x)
+    cells[ci] = make_cell<T>(vol, n, (int)(ci % nc) - 1, (int)((ci / nc) % nc) - 1, (int)(ci / (nc * nc)) - 1);
+}
+// The same cells as bricks.
+template <typename T>
+__global__ void k_build_bricks(const float* __restrict__ vol, int n, CellT<T>* __restrict__ cells) {
+  const long total = brick_cells(n);
+  const long row = brick_row(n), slab = brick_slab(n);
   for (long ci = blockIdx.x * (long)blockDim.x + threadIdx.x; ci < total; ci += (long)gridDim.x * blockDim.x) {
-    const int i = (int)(ci % nc) - 1, j = (int)((ci / nc) % nc) - 1, k = (int)(ci / (nc * nc)) - 1;
-    float v[8];
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      const int x = i + (q & 1), y = j + ((q >> 1) & 1), z = k + ((q >> 2) & 1);
-      v[q] = (x >= 0 && y >= 0 && z >= 0 && x < n && y < n && z < n) ? vol[((long)z * n + y) * n + x] : 0.f;
-    }
-    CellT<T> c;
-    if constexpr (sizeof(T) == 4) {
-      reinterpret_cast<CellT<float>&>(c).lo = make_float4(v[0], v[1], v[2], v[3]);
-      reinterpret_cast<CellT<float>&>(c).hi = make_float4(v[4], v[5], v[6], v[7]);
-    } else {
-      __nv_bfloat162* p = reinterpret_cast<__nv_bfloat162*>(&reinterpret_cast<CellT<__nv_bfloat16>&>(c).v);
-#pragma unroll
-      for (int q = 0; q < 4; ++q) p[q] = __floats2bfloat162_rn(v[2 * q], v[2 * q + 1]);
-    }
-    cells[ci] = c;
+    const int Z = 2 * (int)(ci / slab) + (int)((ci >> 1) & 1), X = (int)(ci % slab / row);
+    const int Y = 2 * (int)(ci % row / 4) + (int)(ci & 1);
+    cells[ci] = make_cell<T>(vol, n, X - 1, Y - 1, Z - 1);
   }
+}
+static __global__ void k_mask_tiles(const float* __restrict__ mask, int n, float* __restrict__ tiles) {
+  const int total = n * n * n;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x)
+    tiles[mask_tile_index(n, i % n, (i / n) % n, i / (n * n))] = mask[i];
 }
 
 struct EvalItem {
@@ -179,11 +188,12 @@ struct SearchChunkArgs {
   const DevParticle* parts;
   const DevRef* refs;
   const double* dmat;        // [norient][9] column-major defineMatrix([phi,theta,psi-phi],'inv')
-  float2* s1;                // [E][ky][part][lpos(z)][TPB_K] slabs, S1_EVAL per evaluation
+  float2* s1;                // [E][ky][z][column], S1_EVAL per evaluation
   float2* s2;                // [E][w][lpos(ky)][PC] planes, S2_PLANE each
   EvalStats* stats;          // [E]
   unsigned long long* keys;  // [E]
   int n_items;
+  int planes;                // z-planes per pass-A CTA
   int radius;
   int interp;
   // With `done` set, the last pass-C CTA of an evaluation decodes it into results / best_keys
@@ -223,31 +233,58 @@ __device__ __forceinline__ void decode_eval(const SearchChunkArgs& a, int n, int
   }
 }
 
-// Sampling matrix rows of RotMat' with RotMat = prior * D (FP64 composition).
-__device__ __forceinline__ void compose_sampling_matrix(const double* prior, const double* d, float m[9]) {
-#pragma unroll
-  for (int i = 0; i < 3; ++i)
-#pragma unroll
-    for (int j = 0; j < 3; ++j) {
-      // RotMat(j, i) = sum_k prior(j, k) D(k, i)
-      double acc = 0.0;
-#pragma unroll
-      for (int k = 0; k < 3; ++k) acc = fma(prior[j + 3 * k], d[k + 3 * i], acc);
-      m[3 * i + j] = (float)acc;
-    }
+// z-planes per pass-A CTA: 1, 2, 4 or 8 at 64^3, up to 4 at 96^3, up to 2 at 128^3.
+__host__ __device__ constexpr bool planes_allowed(int N, int g) {
+  return (g == 1 || g == 2 || g == 4 || g == 8) && g <= (N <= 64 ? 8 : N <= 96 ? 4 : 2);
 }
 
-// Default planes per pass-A CTA; the autotuner of search.cu may pick another supported value.
-__host__ __device__ constexpr int default_planes(int N) { return N <= 64 ? 4 : (N <= 96 ? 2 : 1); }
-
-template <int N, int GG = 0>
+// The line transforms of passes A and B split N = 8 R2: with n = j + R2 r and k = k1 + 8 k2,
+//   X(k) = DFT_R2 over j of [ w_N^(j k1) DFT_8 over r of x(j + R2 r) ],
+// so a thread holds one 8-point or one R2-point butterfly of its own line, neighbouring threads hold
+// neighbouring lines (shared memory is read and written in consecutive words, whatever the axis), all
+// threads of a warp use the same twiddles, and between the two stages the data crosses shared memory
+// once, in place: the R2-point stage reads and writes the slots (k1, 0 .. R2-1) that no other thread
+// touches.  (Teams of 8 lanes transforming one line each crossed it three to four times per axis.)
+template <int N>
 struct SearchCfg {
   static constexpr int NH = N / 2 + 1;
   static constexpr int P = team_size(N);
-  static constexpr int G = GG ? GG : default_planes(N);  // planes per pass-A CTA
-  static constexpr int NT_A = 256;
-  static constexpr int TEAMS_A = NT_A / P;
-  // Pass C uses half as many teams as the y transforms have lines (two rounds of y lines), so
+  static constexpr int R2 = N / 8;
+  // ---- pass A.  A plane's lines are its N/2 row pairs (y, y + N/2) along x, then its N/2 columns along
+  // y (columns 0 and N/2, both real after x, share one).  Element (k1, m) of line q lives at
+  // k1 XA + m XB + q: with XB = 8 and XA = 1 (mod 16 slots of 8 bytes) a half-warp falls on distinct
+  // banks in the gather's patches (8 q x 2 m) and in the y stages, whose sixteen neighbouring columns
+  // kx read slots (kx mod 8, kx / 8) or their mirrors.
+  static constexpr int Q = N / 2;
+  static constexpr int XB = Q + 8;
+  static constexpr int XA = R2 * XB + 1;
+  static_assert(XB % 16 == 8 && XA % 16 == 1 && Q % 8 == 0, "bank layout");
+  static constexpr int NT_A = N == 96 ? 192 : 256;
+  static constexpr int JA = NT_A / Q;            // butterflies of a line formed side by side
+  static_assert(NT_A % Q == 0 && R2 % JA == 0 && 8 % JA == 0 && JA % 4 == 0, "whole rounds and patches");
+  static constexpr size_t SMEM_A = sizeof(float2) * (8 * (size_t)XA + N + N);
+  // resident pass-A CTAs asked of the compiler
+    // Cells in flight per thread (2 UNROLL_A) against resident warps: at 64^3 two and four CTAs per SM
+  // (1,095 ns per evaluation; four and three CTAs 1,150), at 96^3 and 128^3 four (3,490 and 9,180 ns;
+  // two: 3,760 and 10,760).  Four at one CTA more spill and lose by a third: local memory shares the
+  // L1 that the gather streams through.
+  static constexpr int UNROLL_A = N == 64 ? 1 : 2;
+  static constexpr int MINB_A = N <= 96 ? 4 : 2;
+  // ---- pass B: the z lines of one ky, the R2-point stage first (its inputs come straight from global
+  // memory) and the 8-point one second, so that the product needs 8 spectrum and weight elements per
+  // butterfly.  S1 rows hold column N/2 first, then 0 .. N/2-1, padded to whole 32-byte sectors;
+  // element (k1, j) of column c lives at k1 ZA + j TP + c, and thread t has column t % TP, so that both
+  // stages' accesses are consecutive in t.
+  static constexpr int TP = (NH + 3) / 4 * 4;
+  static constexpr int JB = N == 64 ? 8 : 4;
+  static constexpr int NT_B = (TP * JB + 31) / 32 * 32;
+  static constexpr int ZA = 8 * TP + (16 - (7 * TP) % 16) % 16;
+  static_assert((ZA - TP) % 16 == 0 && R2 % JB == 0 && 8 % JB == 0, "bank layout, whole rounds");
+  static constexpr int EVALS_B = N <= 96 ? 4 : 2;
+  static constexpr int MINB_B = N == 128 ? 2 : 3;
+  static constexpr size_t SMEM_B = sizeof(float2) * (R2 * (size_t)ZA + N);
+  static constexpr size_t S1_EVAL = (size_t)N * N * TP;
+  // ---- pass C uses half as many teams as the y transforms have lines (two rounds of y lines), so
   // that the C2R phase, where (2 r + 1 + 1) / 2 row pairs (8 at r = 7) keep as many teams busy,
   // leaves fewer idle and more CTAs fit per SM: 64^3 20 teams of 8 lanes, six CTAs per SM at 64
   // registers (88.7 us per 602-evaluation chunk against 131.1 with 33 teams); 96^3 28 teams and
@@ -259,64 +296,8 @@ struct SearchCfg {
   // contiguous line buffer LP slots; LP = 8 (mod 16) puts neighbouring teams 16 banks apart.
   static constexpr int PY = padded_len(N);
   static constexpr int LP = PY + ((8 - PY % 16) + 16) % 16;
-  // teams with a line buffer for the row-pair transforms (pass A R2C, pass C C2R); the others
-  // idle during those loops, which keeps two pass-A CTAs per SM for every box size
-  static constexpr int TEAMS_LA = N <= 64 ? TEAMS_A : 16;
   static constexpr int TEAMS_LC = 16;  // (2 r + 1 + 1) / 2 <= 16 row pairs for r <= 15
   static_assert(TEAMS_BC >= TEAMS_LC, "pass C needs a team for every line buffer");
-  // Plane pitch of pass A (float2): nh rounded up to even.  With the even pitch the y transform's
-  // teams take consecutive columns, the row-pair R2C's four teams of a warp take the pairs
-  // q, q+2, q+1, q+3 of a group of four, and a bank model of every access puts each half-warp's
-  // two teams on complementary banks in the R2C's reads and writes and in every y-transform stage
-  // (64^3: 512 -> 256 R2C wavefronts per CTA; 96^3 / 128^3 also 3456 -> 2016 / 4096 -> 2560 in the
-  // y transform); the slab store then reads column pairs as 16-byte words.
-  static constexpr int PA = NH + (NH & 1);
-  static constexpr size_t SMEM_A = sizeof(float2) * ((size_t)G * PY * PA + (size_t)TEAMS_LA * LP + N) + 64;
-  // resident pass-A CTAs per SM that shared memory allows (228 KB per SM, 1 KB reserved per CTA),
-  // and the target the register budget is capped for: 5 at 64^3 with one plane per CTA (48
-  // registers, a 12-byte spill; 863.7 us per 602-evaluation chunk against 875.2 at the compiler's
-  // 64 registers and 4 CTAs), none for the multi-plane 64^3 tilings, 2 for the larger boxes, whose
-  // FFT codelets need more registers
-  static constexpr int SMEM_CTAS_A = (int)((228 * 1024) / (SMEM_A + 1024));
-  static constexpr int MINB_A = N <= 64 ? (G == 1 ? 5 : 0) : (SMEM_CTAS_A < 2 ? SMEM_CTAS_A : 2);
-  // Pass B: a CTA transforms the z lines of one ky and one of KS_B parts of the kx columns (NHB
-  // columns at most).  128^3 splits the columns in two: with the whole ky row a CTA needed 544
-  // threads and 95 registers (one CTA per SM, latency-bound); half rows fit three per SM.  At 96^3
-  // two parts (four CTAs per SM instead of two) took pass B from 494 to 448 us per chunk, but pass A's
-  // stores of the second part, which starts at an odd column, from 965 to 1035 us.
-  // Pass A writes S1 as pass B's shared-memory tiles: per (evaluation, ky, column part) a slab of PY
-  // rows (row z at lpos<1>(z)) of TPB_K float2, which pass B fetches with one bulk copy.  The
-  // particle spectrum and weight rows (the caller's layout) come in 16-byte cp.async pieces from the
-  // 16-byte boundary at or below each row start, into rows of even pitch (QP_K float2, WP_K floats),
-  // and are read at the row's offset from that boundary (the same for every row of a CTA: a z step
-  // is N NH elements, a multiple of 16 bytes).  The teams of a warp take consecutive columns: with
-  // the even tile pitch the two teams of a half-warp fall on complementary banks in every stage at
-  // 64^3 (96^3 and 128^3 keep the few conflicts their radix-3 / radix-16 stages had with an odd
-  // pitch), and the four of a warp read the weight rows (pitch WP_K) on disjoint banks.
-  static constexpr int KS_B = N >= 128 ? 2 : 1;
-  static constexpr int NHB = (NH + KS_B - 1) / KS_B;
-  static constexpr int NT_B = ((NHB * P + 31) / 32) * 32;
-  static constexpr int TEAMS_B = NT_B / P;
-  static constexpr int GRID_BX = N * KS_B;
-  // evaluations per pass-B CTA (grid y = ceil(items / EVALS_B)): four at 64^3 and 96^3, two at
-  // 128^3, where the later ones reuse the particle's spectrum (and weight) rows (64^3: pass B 321.5 ->
-  // 309.9 us per 534-evaluation chunk with two, 302.1 with four; 96^3, 69 registers, still two CTAs
-  // per SM: 493.4 -> 505.6 us per 167-evaluation chunk with two, 485.3 with four; 128^3, 56
-  // registers, three CTAs per SM: 446.4 -> 432.6 us per 72-evaluation chunk with two, 436.6 with
-  // four).  A second slab tile, the next evaluation's slab copied while the current one is
-  // transformed (66 KB, three CTAs per SM), took pass B from 295.6 to 307.0 us and the overlapped
-  // 64^3 run from 620 to 679 ms: pass A of the other chunk no longer fits beside three such CTAs.
-  static constexpr int EVALS_B = N <= 96 ? 4 : 2;
-  static constexpr int TPB_K = NHB + 1 + (NHB + 1) % 2;                 // >= NHB + 1, even
-  static constexpr int QP_K = TPB_K;
-  static constexpr int WP_K = ((NHB + 3 + 3) / 4) * 4;                   // >= NHB + 3, 16-byte rows
-  // The weight rows are copied too up to 96^3; at 128^3 the weight is read from L2 when the product
-  // is formed, so that three CTAs per SM fit in shared memory instead of two.
-  static constexpr bool PREF_W = N <= 96;
-  // S1 elements per evaluation: a slab per (ky, column part)
-  static constexpr size_t S1_EVAL = (size_t)N * KS_B * PY * TPB_K;
-  static constexpr size_t SMEM_B = sizeof(float2) * ((size_t)PY * TPB_K + (size_t)N * QP_K + N) +
-                                   (PREF_W ? sizeof(float) * (size_t)N * WP_K : 0);
   // Pass C's tile: S2 planes are written by pass B in this layout (rows ky at lpos<1>(ky), even
   // pitch PC), so pass C brings a plane in with one bulk copy; its y transforms then take
   // consecutive columns (a bank model gives the same wavefronts as the odd pitch with paired
@@ -326,7 +307,7 @@ struct SearchCfg {
   static constexpr size_t SMEM_C = sizeof(float2) * (S2_PLANE + N + (size_t)TEAMS_LC * LP);
 };
 
-// S1 elements per evaluation of box n (slabs padded to the z pass's tiles).
+// S1 elements per evaluation of box n.
 inline size_t s1_eval_elems(int n) {
   return n == 64 ? SearchCfg<64>::S1_EVAL : n == 96 ? SearchCfg<96>::S1_EVAL : SearchCfg<128>::S1_EVAL;
 }
@@ -349,439 +330,460 @@ __device__ __forceinline__ Tv block_sum(Tv v, Tv* red) {
   return t;  // valid in thread 0
 }
 
-// Gather of the G planes of pass A through corner cells.  Each warp takes RU whole rows per step;
-// lane l samples x = l + 32 k (k < N / 32) of each, so one load instruction of a warp covers 32
-// consecutive voxels of a row (neighbouring cells, few L1 lines per request).  A thread computes
-// its sample point once per row and steps 32 voxels along x by adding 32 x (first column of the
-// sampling matrix); its RU * N / 32 cell loads are all issued before any is used.  Sums of r and
-// r^2 are formed per step in FP32 and accumulated in FP64.
-// A lane whose voxel lies outside its row's mask extent (mask_rows) skips its cell: it reads cell 0,
-// which every such lane of the warp shares, and its value is 0 as the mask would make it.
-template <int N, typename T, int MODE, int GG>
-__device__ __forceinline__ void gather_cells(const CellT<T>* __restrict__ cells, const float* __restrict__ mask,
-                                             const unsigned* __restrict__ mask_rows, const float m[9], float tx,
-                                             float ty, float tz, int z0, float* __restrict__ fplanes, double& s1,
-                                             double& s2) {
-  using C = SearchCfg<N, GG>;
-  constexpr int G = C::G, NT = C::NT_A;
-  constexpr int SEG = N / 32;                     // row segments per lane
-  constexpr int RU = SEG >= 3 ? 2 : 4 / SEG;      // rows per warp per step: U = RU * SEG loads in flight
-  // (two rows at 96^3 / 128^3: 6 / 8 cells in flight; 128^3 pass A 149 us per 9 evaluations from 156)
-  constexpr int U = RU * SEG;
-  constexpr int WARPS = NT / 32;
-  constexpr int ROWS = G * N;
-  static_assert(N % 32 == 0 && ROWS % (WARPS * RU) == 0, "gather tiling");
-  constexpr int c = N / 2;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const float step_x = 32.f * m[0], step_y = 32.f * m[3], step_z = 32.f * m[6];
-#pragma unroll 1
-  for (int r0 = warp * RU; r0 < ROWS; r0 += WARPS * RU) {
-    CellT<T> cv[U];
-    float fr[U][3];
-    bool ok[U];
-    float mk[U];
-#pragma unroll
-    for (int ru = 0; ru < RU; ++ru) {
-      const int row = r0 + ru, y = row % N, zl = row / N, z = z0 + zl;
-      const unsigned ext = mask_rows ? __ldg(mask_rows + z * N + y) : ((unsigned)N << 16);
-      const int lo = (int)(ext & 0xffffu), hi = (int)(ext >> 16);
-      const float pu = (float)(lane - c) - tx, pv = (float)(y - c) - ty, pw = (float)(z - c) - tz;
-      float sx = fmaf(m[0], pu, fmaf(m[1], pv, m[2] * pw)) + (float)c;
-      float sy = fmaf(m[3], pu, fmaf(m[4], pv, m[5] * pw)) + (float)c;
-      float sz = fmaf(m[6], pu, fmaf(m[7], pv, m[8] * pw)) + (float)c;
-#pragma unroll
-      for (int k = 0; k < SEG; ++k) {
-        const int u = ru * SEG + k;
-        const int x = lane + 32 * k;
-        const bool in = x >= lo && x < hi;
-        unsigned ci = cell_index_gather<MODE>(N, sx, sy, sz, fr[u], ok[u]);
-        ci = in ? ci : 0u;
-        ok[u] = ok[u] && in;
-        cv[u] = load_cell(cells + ci);
-        mk[u] = !mask ? 1.f : (in ? __ldg(mask + ((long)z * N + y) * N + x) : 0.f);
-        sx += step_x;
-        sy += step_y;
-        sz += step_z;
-      }
-    }
-    float p1 = 0.f, p2 = 0.f;
-#pragma unroll
-    for (int ru = 0; ru < RU; ++ru) {
-      const int row = r0 + ru, y = row % N, zl = row / N;
-      float* dst = fplanes + ((size_t)zl * C::PY + lpos<1>(y)) * (2 * C::PA) + lane;
-#pragma unroll
-      for (int k = 0; k < SEG; ++k) {
-        const int u = ru * SEG + k;
-        float cvv[8];
-        cell_values(cv[u], cvv);
-        const float val = (ok[u] ? cell_trilinear(cvv, fr[u]) : 0.f) * mk[u];
-        dst[32 * k] = val;
-        p1 += val;
-        p2 = fmaf(val, val, p2);
-      }
-    }
-    s1 += (double)p1;
-    s2 += (double)p2;
-  }
+// max of |a|, |b|, |c|; NaN when any is NaN.
+__device__ __forceinline__ float max_abs_nan(float a, float b, float c) {
+  float d;
+  asm("{\n .reg .f32 x, y, z;\n abs.f32 x, %1;\n abs.f32 y, %2;\n abs.f32 z, %3;\n max.NaN.f32 x, x, y;\n"
+      " max.NaN.f32 %0, x, z;\n}\n"
+      : "=f"(d)
+      : "f"(a), "f"(b), "f"(c));
+  return d;
+}
+
+// Cell load under a predicate; an inactive lane's value is undefined and its access is not made.
+__device__ __forceinline__ CellT<float> load_cell_if(const CellT<float>* p, bool on) {
+  CellT<float> c;
+  asm volatile("{\n .reg .pred q;\n setp.ne.s32 q, %9, 0;\n"
+      " @q ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n}\n"
+      : "=f"(c.lo.x), "=f"(c.lo.y), "=f"(c.lo.z), "=f"(c.lo.w), "=f"(c.hi.x), "=f"(c.hi.y), "=f"(c.hi.z),
+        "=f"(c.hi.w)
+      : "l"(p), "r"((int)on));
+  return c;
+}
+__device__ __forceinline__ CellT<__nv_bfloat16> load_cell_if(const CellT<__nv_bfloat16>* p, bool on) {
+  CellT<__nv_bfloat16> c;
+  asm volatile("{\n .reg .pred q;\n setp.ne.s32 q, %5, 0;\n @q ld.global.nc.v4.u32 {%0, %1, %2, %3}, [%4];\n}\n"
+      : "=r"(c.v.x), "=r"(c.v.y), "=r"(c.v.z), "=r"(c.v.w)
+      : "l"(p), "r"((int)on));
+  return c;
+}
+
+// Same interpolation order as sample_linear, so both paths give identical results.
+__device__ __forceinline__ float cell_trilinear(const float v[8], const float f[3]) {
+  const float c00 = fmaf(f[0], v[1] - v[0], v[0]), c10 = fmaf(f[0], v[3] - v[2], v[2]);
+  const float c01 = fmaf(f[0], v[5] - v[4], v[4]), c11 = fmaf(f[0], v[7] - v[6], v[6]);
+  const float c0 = fmaf(f[1], c10 - c00, c00), c1 = fmaf(f[1], c11 - c01, c01);
+  return fmaf(f[2], c1 - c0, c0);
+}
+
+// Sampling point of voxel (x, y, z) under the matrix rows m, and the reference's value there, for
+// the modes without cells.
+template <typename T>
+__device__ __noinline__ float sample_any(int mode, const T* __restrict__ src, int n, const float* __restrict__ m,
+                                         float u, float v, float w) {
+  const float c = (float)(n / 2);
+  return sample(mode, src, n, n, n, fmaf(m[0], u, fmaf(m[1], v, m[2] * w)) + c,
+                fmaf(m[3], u, fmaf(m[4], v, m[5] * w)) + c, fmaf(m[6], u, fmaf(m[7], v, m[8] * w)) + c);
 }
 
 // ------------------------------------------------------------------ pass A
-template <int N, typename T, int GG = 0>
-__global__ void __launch_bounds__(SearchCfg<N, GG>::NT_A, SearchCfg<N, GG>::MINB_A) k_search_fwd_xy(const SearchChunkArgs a,
-                                                                           const float2* __restrict__ g_tw) {
-  using C = SearchCfg<N, GG>;
-  constexpr int NH = C::NH, G = C::G, P = C::P;
+// One z-plane after another: thread (q, j) samples the voxels x = j + R2 r (r = 0..7) of rows q and
+// q + N/2, whose pairs are the inputs of its first x butterfly, so the rotated plane crosses shared
+// memory only in the thread's own slots.  A warp takes 8 rows x 4 columns of the plane and reads the
+// cells from bricks (see brick_index); floors by a round-down addition (kFloorMagic).
+//
+// CELLS: the two trilinear modes through the cells; else any mode from the plain volume (tricubic, or
+// a caller without cells), its sampler a call.
+template <int N, typename T, bool CELLS>
+__global__ void __launch_bounds__(SearchCfg<N>::NT_A, SearchCfg<N>::MINB_A) k_search_fwd_xy(
+    const SearchChunkArgs a, const float2* __restrict__ g_tw) {
+  using C = SearchCfg<N>;
+  constexpr int R2 = C::R2, Q = C::Q, XA = C::XA, XB = C::XB, JA = C::JA;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  constexpr int PY = C::PY, LP = C::LP;
-  constexpr int PA = C::PA;
-  float2* planes = reinterpret_cast<float2*>(smem_raw);          // [G][PY][PA], row y at lpos<1>(y)
-  float2* lines = planes + (size_t)G * PY * PA;                   // [TEAMS][LP]
-  float2* s_tw = lines + (size_t)C::TEAMS_LA * LP;                 // [N]
-  float* s_m = reinterpret_cast<float*>(s_tw + N);                // 9 floats
+  float2* buf = reinterpret_cast<float2*>(smem_raw);  // [8][XA]
+  float2* s_tw = buf + 8 * XA;                         // [N]
+  float2* s_col = s_tw + N;                            // [N], the packed columns 0 and N/2 after y
+  __shared__ float s_m[9];
   __shared__ double red[2][32];
 
   const int e = blockIdx.y;
   if (e >= a.n_items) return;
-  const int z0 = blockIdx.x * G;
   const EvalItem it = a.items[e];
   const DevParticle& pt = a.parts[it.particle];
   const DevRef rf = a.refs[pt.ref];
-  const T* __restrict__ src = reinterpret_cast<const T*>(rf.data);
-  const float* __restrict__ mask = rf.mask;
-
   load_twiddles<N>(s_tw, g_tw);
-  if (threadIdx.x == 0) compose_sampling_matrix(pt.prior, a.dmat + 9L * it.orient, s_m);
-  __syncthreads();
-  float m[9];
+  if (threadIdx.x < 9) {
+    // sampling matrix rows of RotMat' with RotMat = prior * D (FP64 composition): entry (i, j) is
+    // RotMat(j, i) = sum_k prior(j, k) D(k, i)
+    const int i = threadIdx.x / 3, j = threadIdx.x % 3;
+    const double* d = a.dmat + 9L * it.orient;
+    double acc = 0.0;
 #pragma unroll
-  for (int i = 0; i < 9; ++i) m[i] = s_m[i];
-  const float tx = pt.shift[0], ty = pt.shift[1], tz = pt.shift[2];
+    for (int k = 0; k < 3; ++k) acc = fma(pt.prior[j + 3 * k], d[k + 3 * i], acc);
+    s_m[threadIdx.x] = (float)acc;
+  }
+  __syncthreads();
+  const bool weighted = rf.wref || pt.wedge;
+  const CellT<T>* __restrict__ cells = reinterpret_cast<const CellT<T>*>(rf.bricks);
+  // samples with |s - (N-1)/2| <= lim on every axis are inside (0 <= s <= N-1, or -1 < s < N)
+  constexpr float h = 0.5f * (N - 1);
+  const float lim = a.interp == EMC_INTERP_LINEAR_BORDER ? __int_as_float(__float_as_int(h + 1.f) - 1) : h;
+  const int q = threadIdx.x % Q, jt = threadIdx.x / Q;
   constexpr int c = N / 2;
+  // shared-memory column of the y stages: kx = q, its mirror N - kx (N/2 for the packed column 0)
+  const int mir = q == 0 ? Q : N - q;
+  const int slot_k = (q & 7) * XA + (q >> 3) * XB, slot_m = (mir & 7) * XA + (mir >> 3) * XB;
+  float sum1 = 0.f, sum2 = 0.f;
+  // first x stage of a butterfly whose inputs lie in this thread's slots, in place
+  auto first_x_stage = [&](float2* own) {
+    float2 v[8];
+#pragma unroll
+    for (int r = 0; r < 8; ++r) v[r] = own[r * XA];
+    Dft<8, -1>::run(v);
+#pragma unroll
+    for (int r = 0; r < 8; ++r) own[r * XA] = v[r];
+  };
 
-  // 1. gather (x fastest: a warp walks 32 consecutive voxels of one row)
-  double s1 = 0.0, s2 = 0.0;
-  float* fplanes = reinterpret_cast<float*>(planes);
-  if (rf.cells && a.interp == EMC_INTERP_LINEAR) {
-    gather_cells<N, T, EMC_INTERP_LINEAR, GG>(reinterpret_cast<const CellT<T>*>(rf.cells), mask, rf.mask_rows, m, tx,
-                                              ty, tz, z0, fplanes, s1, s2);
-  } else if (rf.cells && a.interp == EMC_INTERP_LINEAR_BORDER) {
-    gather_cells<N, T, EMC_INTERP_LINEAR_BORDER, GG>(reinterpret_cast<const CellT<T>*>(rf.cells), mask, rf.mask_rows,
-                                                     m, tx, ty, tz, z0, fplanes, s1, s2);
-  } else {
-    for (int idx = threadIdx.x; idx < G * N * N; idx += C::NT_A) {
-      const int x = idx % N, y = (idx / N) % N, zl = idx / (N * N);
-      const int z = z0 + zl;
-      const float u = (float)(x - c) - tx, v = (float)(y - c) - ty, w = (float)(z - c) - tz;
-      const float sx = fmaf(m[0], u, fmaf(m[1], v, m[2] * w)) + (float)c;
-      const float sy = fmaf(m[3], u, fmaf(m[4], v, m[5] * w)) + (float)c;
-      const float sz = fmaf(m[6], u, fmaf(m[7], v, m[8] * w)) + (float)c;
-      float val = sample(a.interp, src, N, N, N, sx, sy, sz);
-      if (mask) val *= __ldg(mask + ((long)z * N + y) * N + x);
-      fplanes[((size_t)zl * PY + lpos<1>(y)) * (2 * PA) + x] = val;
-      s1 += (double)val;
-      s2 += (double)val * (double)val;
+#pragma unroll 1
+  for (int z = blockIdx.x * a.planes; z < (int)(blockIdx.x + 1) * a.planes; ++z) {
+    // 1. gather and the first x stage, rows gq and gq + N/2
+    {
+      const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+      const int gq = (lane & 7) + 8 * (warp % (Q / 8)), gj = (lane >> 3) + 4 * (warp / (Q / 8));
+      const float tx = pt.shift[0], pw = (float)(z - c) - pt.shift[2];
+      const float pva = (float)(gq - c) - pt.shift[1], pvb = (float)(gq + Q - c) - pt.shift[1];
+      if constexpr (CELLS) {
+        constexpr int U = C::UNROLL_A;
+        float base[2][3], mx[3];  // sample points at u = 0 of the two rows
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+          const float w = s_m[3 * i + 2] * pw;
+          base[0][i] = fmaf(s_m[3 * i + 1], pva, w) + (float)c;
+          base[1][i] = fmaf(s_m[3 * i + 1], pvb, w) + (float)c;
+          mx[i] = s_m[3 * i];
+        }
+        // the rows' x extents of non-zero mask voxels: the samples outside need no cell
+        int lo[2], len[2];
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+          const unsigned ext = rf.mask_rows ? __ldg(rf.mask_rows + z * N + gq + k * Q) : (unsigned)N << 16;
+          lo[k] = (int)(ext & 0xffffu);
+          len[k] = (int)(ext >> 16) - lo[k];
+        }
+        const float* mask = rf.mask_tiles ? rf.mask_tiles + mask_tile_index(N, lane >> 3, gq, z) : nullptr;
+#pragma unroll 1
+        for (int j = gj; j < R2; j += JA) {
+          // U r (2 U cells in flight) per step, the samples left in the thread's own slots: a rolled
+          // loop, since the compiler otherwise starts all sixteen loads at once and spills
+          float2* own = buf + j * XB + gq;
+          float xj = (float)(j - c);
+          int x = j;
+#pragma unroll 1
+          for (int r0 = 0; r0 < 8; r0 += U, x += U * R2, xj += (float)(U * R2), own += U * XA) {
+            CellT<T> cell[U][2];
+            float f[U][2][3], mk[U][2];
+            bool ok[U][2];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+              const float pu = (xj + (float)(R2 * u)) - tx;
+#pragma unroll
+              for (int k = 0; k < 2; ++k) {
+                float off[3];
+                unsigned cc[3];
+#pragma unroll
+                for (int i = 0; i < 3; ++i) {
+                  const float s = fmaf(mx[i], pu, base[k][i]);
+                  const float fl = __fadd_rd(s, kFloorMagic);
+                  f[u][k][i] = s - (fl - kFloorMagic);
+                  off[i] = s - h;
+                  cc[i] = __float_as_uint(fl) + (1u - kFloorBits);
+                }
+                ok[u][k] = max_abs_nan(off[0], off[1], off[2]) <= lim && (unsigned)(x + R2 * u - lo[k]) < (unsigned)len[k];
+                // brick_index(N, X, Y, Z)
+                constexpr unsigned row = brick_row(N), half = brick_slab(N) / 2;
+                const unsigned idx = cc[2] * half - (cc[2] & 1u) * (half - 2u) + cc[0] * row + 2u * cc[1] - (cc[1] & 1u);
+                cell[u][k] = load_cell_if(cells + idx, ok[u][k]);
+                // x / 4 advances the tile row, y / 8 the tile
+                mk[u][k] = mask ? __ldg(mask + ((x + R2 * u) / 4 * (N / 8) + k * (Q / 8)) * 32) : 1.f;
+              }
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+              float val[2];
+#pragma unroll
+              for (int k = 0; k < 2; ++k) {
+                float cv[8];
+                cell_values(cell[u][k], cv);
+                val[k] = ok[u][k] ? cell_trilinear(cv, f[u][k]) * mk[u][k] : 0.f;
+              }
+              own[u * XA] = make_float2(val[0], val[1]);
+              if (!weighted) {
+                sum1 += val[0] + val[1];
+                sum2 = fmaf(val[0], val[0], fmaf(val[1], val[1], sum2));
+              }
+            }
+          }
+          first_x_stage(buf + j * XB + gq);
+        }
+      } else {
+        const T* src = reinterpret_cast<const T*>(rf.data);
+        const long plane = (long)z * N * N;
+#pragma unroll 1
+        for (int j = gj; j < R2; j += JA) {
+#pragma unroll 1
+          for (int r = 0; r < 8; ++r) {
+            const int x = j + R2 * r;
+            const float pu = (float)(x - c) - tx;
+            float va = sample_any(a.interp, src, N, s_m, pu, pva, pw);
+            float vb = sample_any(a.interp, src, N, s_m, pu, pvb, pw);
+            if (rf.mask) {
+              va *= __ldg(rf.mask + plane + (long)gq * N + x);
+              vb *= __ldg(rf.mask + plane + (long)(gq + Q) * N + x);
+            }
+            sum1 += va + vb;
+            sum2 = fmaf(va, va, fmaf(vb, vb, sum2));
+            buf[r * XA + j * XB + gq] = make_float2(va, vb);
+          }
+          first_x_stage(buf + j * XB + gq);
+        }
+      }
+    }
+    __syncthreads();
+    // 2. second x stage: Z(k1 + 8 k2) of every row pair, left at (k1, k2)
+#pragma unroll 1
+    for (int k1 = jt; k1 < 8; k1 += JA) {
+      float2* line = buf + k1 * XA + q;
+      float2 v[R2];
+#pragma unroll
+      for (int m = 0; m < R2; ++m) v[m] = line[m * XB];
+#pragma unroll
+      for (int m = 1; m < R2; ++m) v[m] = cmul(v[m], s_tw[m * k1]);
+      Dft<R2, -1>::run(v);
+#pragma unroll
+      for (int m = 0; m < R2; ++m) line[m * XB] = v[m];
+    }
+    __syncthreads();
+    // 3. first y stage of column kx = q: rows y = j + R2 r from the Hermitian split of the row pairs
+    // y, y + N/2 = (r, r + 4).  Columns 0 and N/2 of a row are real and share a column as (X(0), X(N/2)).
+    // The pairs' entries kx and N - kx are this column's alone: the results go back into them.
+#pragma unroll 1
+    for (int j = jt; j < R2; j += JA) {
+      float2* pk = buf + slot_k + j;
+      float2* pm = buf + slot_m + j;
+      float2 v[8];
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        const float2 zk = pk[R2 * r], zm = pm[R2 * r];
+        if (q == 0) {
+          v[r] = make_float2(zk.x, zm.x);
+          v[r + 4] = make_float2(zk.y, zm.y);
+        } else {
+          v[r] = make_float2(0.5f * (zk.x + zm.x), 0.5f * (zk.y - zm.y));
+          v[r + 4] = make_float2(0.5f * (zk.y + zm.y), -0.5f * (zk.x - zm.x));
+        }
+      }
+      Dft<8, -1>::run(v);
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        pk[R2 * r] = v[r];
+        pm[R2 * r] = v[r + 4];
+      }
+    }
+    __syncthreads();
+    // 4. second y stage, straight to S1 (columns 1 .. N/2-1); the packed column to shared memory
+    float2* s1 = a.s1 + (size_t)e * C::S1_EVAL + (size_t)z * C::TP;
+#pragma unroll 1
+    for (int k1 = jt; k1 < 8; k1 += JA) {
+      const float2* col = buf + (k1 < 4 ? slot_k : slot_m) + R2 * (k1 & 3);
+      float2 v[R2];
+#pragma unroll
+      for (int m = 0; m < R2; ++m) v[m] = col[m];
+#pragma unroll
+      for (int m = 1; m < R2; ++m) v[m] = cmul(v[m], s_tw[m * k1]);
+      Dft<R2, -1>::run(v);
+      if (q == 0) {
+#pragma unroll
+        for (int k2 = 0; k2 < R2; ++k2) s_col[k1 + 8 * k2] = v[k2];
+      } else {
+#pragma unroll
+        for (int k2 = 0; k2 < R2; ++k2) s1[(size_t)(k1 + 8 * k2) * N * C::TP + 1 + q] = v[k2];
+      }
+    }
+    __syncthreads();
+    // columns N/2 and 0 from the packed one: with Z = F(X(0) + i X(N/2)),
+    // F X(0)(y) = (Z(y) + conj Z(-y)) / 2 and F X(N/2)(y) = (Z(y) - conj Z(-y)) / 2i
+    if (threadIdx.x < N) {
+      const float2 zp = s_col[threadIdx.x], zm = s_col[(N - threadIdx.x) % N];
+      *reinterpret_cast<float4*>(s1 + (size_t)threadIdx.x * N * C::TP) =
+          make_float4(0.5f * (zp.y + zm.y), -0.5f * (zp.x - zm.x), 0.5f * (zp.x + zm.x), 0.5f * (zp.y - zm.y));
     }
   }
-  if (!(rf.wref || pt.wedge)) {
-    // E_R from the real-space sums (Parseval) is needed only without a weight on the reference;
-    // with one, pass B forms the weighted spectral energy (the branch is uniform over the block)
-    double t1 = block_sum(s1, red[0]);
-    double t2 = block_sum(s2, red[1]);
+  if (!weighted) {
+    // E_R from the real-space sums (Parseval) is needed only without a weight on the reference; with
+    // one, pass B forms the weighted spectral energy (the branch is uniform over the block)
+    double t1 = block_sum((double)sum1, red[0]);
+    double t2 = block_sum((double)sum2, red[1]);
     if (threadIdx.x == 0) {
       atomicAdd(&a.stats[e].sum_r, t1);
       atomicAdd(&a.stats[e].sum_r2, t2);
     }
   }
-  __syncthreads();
-
-  const int team = threadIdx.x / P, lane = threadIdx.x % P;
-  LineTw<N, P> tc;
-  tc.init(s_tw, lane);
-  // 2. R2C along x: rows 2q and 2q+1 of the slab share one complex FFT
-  {
-    constexpr int NPAIRS = G * N / 2;
-    const bool has_line = team < C::TEAMS_LA;
-    float2* buf = lines + (size_t)(has_line ? team : 0) * LP;
-    static_assert((C::TEAMS_LA * P) % 32 == 0, "line-buffer teams fill whole warps");
-    // warps without line buffers (96^3, 128^3: the second half of the CTA) skip the loop
-    for (int base = 0; base < NPAIRS && threadIdx.x < C::TEAMS_LA * P; base += C::TEAMS_LA) {
-      const int q = base + ((team & ~3) | ((team & 1) << 1) | ((team >> 1) & 1));  // pairs 0, 2, 1, 3
-      const bool active = has_line && q < NPAIRS;
-      // rows 2q, 2q+1 of the slab (same plane, adjacent padded rows since 2q+1 is odd)
-      const int zl = (2 * q) / N, ya = (2 * q) % N;
-      const size_t row_a = (size_t)zl * PY + lpos<1>(ya);
-      const float* ra = fplanes + row_a * (2 * PA);
-      const float* rb = ra + 2 * PA;
-      // the transform's last stage stays in registers: v[b][r] = Z(k), k = lane + b P + NSL r
-      using LS = LastStage<N, P>;
-      float2 v[LS::PER][LS::RL];
-      fft_line_in_regs<N, -1, P, 1>([&](int n) { return make_float2(ra[n], rb[n]); }, buf, 1, lane, s_tw, active,
-                                    &tc, v);
-      // Hermitian split of the two packed rows: Z(N - k) sits on lane (P - lane) mod P of the team,
-      // butterfly block NSL/P - 1 - b, index RL - 1 - r (lane 0 holds its own partners and Z(N/2)).
-      // Columns 0 and N/2 of a row transform are real: row a's pair goes to slot 0 of row a, row
-      // b's to slot 0 of row b, as (X(0), X(N/2)), so the y pass needs N/2 complex lines.
-      constexpr int NB_P = LS::NSL / P;
-      constexpr int JH = (N / 2) % LS::NSL, BH = JH / P, RH = (N / 2) / LS::NSL;
-      static_assert(JH % P == 0 && LS::NSL % P == 0, "Z(N/2) on lane 0");
-      const int wl = threadIdx.x & 31;
-      const int src = (wl & ~(P - 1)) | ((P - lane) & (P - 1));
-      float2* oa = planes + row_a * PA;
-      float2* ob = oa + PA;
-#pragma unroll
-      for (int b = 0; b < LS::PER; ++b) {
-#pragma unroll
-        for (int r = 0; r < LS::RL; ++r) {
-          if (b * P + r * LS::NSL < N / 2) {
-            const float2 sent = v[NB_P - 1 - b][LS::RL - 1 - r];
-            float2 zm = make_float2(__shfl_sync(0xffffffffu, sent.x, src), __shfl_sync(0xffffffffu, sent.y, src));
-            if (lane == 0) {
-              zm = b > 0 ? v[(NB_P - b) % LS::PER][LS::RL - 1 - r] : (r > 0 ? v[0][(LS::RL - r) % LS::RL] : v[BH][RH]);
-            }
-            const float2 zk = v[b][r];
-            const int k = lane + b * P + r * LS::NSL;
-            if (active && k < N / 2) {
-              if (k == 0) {
-                oa[0] = make_float2(zk.x, zm.x);
-                ob[0] = make_float2(zk.y, zm.y);
-              } else {
-                oa[k] = make_float2(0.5f * (zk.x + zm.x), 0.5f * (zk.y - zm.y));
-                ob[k] = make_float2(0.5f * (zk.y + zm.y), -0.5f * (zk.x - zm.x));
-              }
-            }
-          }
-        }
-      }
-      __syncwarp();
-    }
-  }
-  __syncthreads();
-  // 3. FFT along y for columns 0 .. N/2-1 of every plane (column 0 carries X(0) + i X(N/2))
-  {
-    constexpr int NLINES = G * (N / 2);
-    static_assert(NLINES % (32 / P) == 0, "a warp's teams are all active or all idle");
-    for (int base = 0; base < NLINES; base += C::TEAMS_A) {
-      // a warp whose teams all lie past the last line (96^3: the second round) skips the round
-      if (base + (int)(threadIdx.x >> 5) * (32 / P) >= NLINES) continue;
-      const int li = base + team;
-      const bool active = li < NLINES;
-      const int zl = active ? li / (N / 2) : 0, kx = active ? li % (N / 2) : 0;
-      fft_line<N, -1, P, 1>(planes + (size_t)zl * PY * PA + kx, PA, lane, s_tw, active, &tc);
-    }
-  }
-  __syncthreads();
-  // 4. store plane z0 + zl into the S1 slabs (row lpos(z) of slab (ky = y, column part)), values
-  //    gathered from their padded positions; columns 0 and N/2 are separated from the packed
-  //    column 0: with Z = F(X(0) + i X(N/2)),
-  //    F X(0)(y) = (Z(y) + conj Z(-y)) / 2 and F X(N/2)(y) = (Z(y) - conj Z(-y)) / 2i
-  {
-    // F X(kx)(y) of local plane zl: columns 0 and N/2 separated from the packed column 0
-    auto s1_value = [&](int zl, int y, int kx) {
-      const float2* pl = planes + (size_t)zl * PY * PA;
-      if (kx >= NH) return make_float2(0.f, 0.f);
-      if (kx == 0 || kx == NH - 1) {
-        const float2 zp = pl[lpos<1>(y) * PA], zm = pl[lpos<1>((N - y) % N) * PA];
-        return kx == 0 ? make_float2(0.5f * (zp.x + zm.x), 0.5f * (zp.y - zm.y))
-                       : make_float2(0.5f * (zp.y + zm.y), -0.5f * (zp.x - zm.x));
-      }
-      return pl[lpos<1>(y) * PA + kx];
-    };
-    float2* dst = a.s1 + (size_t)e * C::S1_EVAL;
-    {
-      // slabs [ky][part][lpos(z)][TPB_K] (part: columns [part NHB, part NHB + NHB)): whole rows, pad
-      // columns zero, two elements per 16-byte store
-      constexpr int RP = C::TPB_K / 2, KS = C::KS_B, NB = C::NHB;
-      constexpr int NV = G * N * KS * RP;
-      for (int i = threadIdx.x; i < NV; i += C::NT_A) {
-        const int row = i / (KS * RP), rem = i % (KS * RP);  // row = zl * N + y
-        const int part = rem / RP, c = rem % RP;
-        const int zl = row / N, y = row % N;
-        const int k0 = part * NB + 2 * c;
-        float2 v0, v1;
-        if (k0 % 2 == 0 && k0 + 1 < NH - 1 && k0 != 0 && 2 * c + 1 < NB) {
-          // an ordinary column pair: one 16-byte read (even pitch, even column)
-          const float4 q4 = *reinterpret_cast<const float4*>(planes + ((size_t)zl * PY + lpos<1>(y)) * PA + k0);
-          v0 = make_float2(q4.x, q4.y);
-          v1 = make_float2(q4.z, q4.w);
-        } else {
-          v0 = 2 * c < NB ? s1_value(zl, y, k0) : make_float2(0.f, 0.f);
-          v1 = 2 * c + 1 < NB ? s1_value(zl, y, k0 + 1) : make_float2(0.f, 0.f);
-        }
-        *reinterpret_cast<float4*>(dst + (((size_t)y * KS + part) * PY + lpos<1>(z0 + zl)) * C::TPB_K + 2 * c) =
-            make_float4(v0.x, v0.y, v1.x, v1.y);
-      }
-    }
-  }
 }
 
 // ------------------------------------------------------------------ pass B
-// Pass B: pass A left the (evaluation, ky, column part) slab in the tile's
-// layout, so one cp.async.bulk completed on an mbarrier brings it in; the particle spectrum and
-// weight rows arrive meanwhile as 16-byte cp.async pieces, and the fused z lines read them at the
-// rows' offsets from their 16-byte boundaries.  A spectrum or weight whose base is not 16-byte
-// aligned (a caller's buffer at an odd element offset) is copied element by element, at offset 0.
-template <int N>
-__device__ __forceinline__ void z_mul_bulk(const SearchChunkArgs& a, const float2* __restrict__ g_tw) {
-  using C = SearchCfg<N>;
-  constexpr int NH = C::NH, P = C::P, NT = C::NT_B, NB = C::NHB, TP = C::TPB_K, QP = C::QP_K, WP = C::WP_K;
-  static_assert(C::TEAMS_B >= NB, "one round of z lines");
-  constexpr unsigned SLAB_BYTES = (unsigned)(sizeof(float2) * C::PY * TP);
-  static_assert(SLAB_BYTES % 16 == 0, "bulk copy size");
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  float2* tile = reinterpret_cast<float2*>(smem_raw);                // [PY][TP], row z at lpos<1>(z)
-  float2* s_q = tile + (size_t)C::PY * TP;                            // [N][QP]
-  float* s_w = reinterpret_cast<float*>(s_q + (size_t)N * QP);       // [N][WP] (PREF_W)
-  float2* s_tw = reinterpret_cast<float2*>(s_w + (C::PREF_W ? (size_t)N * WP : 0));  // [N]
-  __shared__ double red[32];
-  __shared__ uint64_t bar;
+// Outputs 0 and R - 1 of an inverse R-point transform; tw8: w_N^(8 k) = e^(-2 pi i k / R) at index 8 k.
+template <int R>
+__device__ __forceinline__ void idft_ends(const float2 v[R], const float2* tw8, float2& first, float2& last) {
+  float2 s[R / 2], d[R / 2];
+#pragma unroll
+  for (int k = 0; k < R / 2; ++k) {
+    s[k] = cadd(v[k], v[k + R / 2]);
+    d[k] = csub(v[k], v[k + R / 2]);  // e^(-2 pi i k / R) changes sign from k to k + R / 2
+  }
+  if constexpr (R == 8) {
+    first = cadd(cadd(s[0], s[2]), cadd(s[1], s[3]));
+    const float2 p = csub(d[1], d[3]), t = cadd(d[1], d[3]);  // e^(-i pi/4) d1 + e^(-3 i pi/4) d3
+    last.x = d[0].x + d[2].y + EMC_SQRT1_2 * (p.x + t.y);
+    last.y = d[0].y - d[2].x + EMC_SQRT1_2 * (p.y - t.x);
+  } else {
+    float2 s0 = cadd(s[0], s[1]), s1 = cadd(s[2], s[3]), e0 = d[0], e1 = cmul(d[1], tw8[8]);
+#pragma unroll
+    for (int k = 4; k < R / 2; k += 2) {
+      s0 = cadd(s0, s[k]);
+      s1 = cadd(s1, s[k + 1]);
+    }
+#pragma unroll
+    for (int k = 2; k < R / 2; k += 2) {
+      e0 = cadd(e0, cmul(d[k], tw8[8 * k]));
+      e1 = cadd(e1, cmul(d[k + 1], tw8[8 * (k + 1)]));
+    }
+    first = cadd(s0, s1);
+    last = cadd(e0, e1);
+  }
+}
 
-  // EVALS_B consecutive evaluations of the chunk (consecutive orientations of one particle, but at
-  // a particle boundary): the spectrum and weight rows are copied again only when the particle changes
+// The z lines of one ky for EVALS_B consecutive evaluations (consecutive orientations of one
+// particle, but at a particle boundary).  A butterfly's spectrum and weight elements are asked for a
+// stage before its product needs them; at 64^3, where a thread has one butterfly, they stay in
+// registers while the particle does not change.
+template <int N>
+__global__ void __launch_bounds__(SearchCfg<N>::NT_B, SearchCfg<N>::MINB_B) k_search_z_mul(
+    const SearchChunkArgs a, const float2* __restrict__ g_tw) {
+  using C = SearchCfg<N>;
+  constexpr int R2 = C::R2, TP = C::TP, ZA = C::ZA, JB = C::JB, NH = C::NH;
+  constexpr bool ONE = JB == R2;  // one butterfly of the second stage per thread
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  float2* buf = reinterpret_cast<float2*>(smem_raw);  // [R2][ZA]
+  float2* s_tw = buf + R2 * ZA;                        // [N]
+  __shared__ double red[32];
   const int e_first = blockIdx.y * C::EVALS_B;
   if (e_first >= a.n_items) return;
   const int ne = min(C::EVALS_B, a.n_items - e_first);
-  // this CTA's columns: kx in [k0, k0 + cnt)
-  const int ky = blockIdx.x / C::KS_B;
-  const int k0 = (int)(blockIdx.x % C::KS_B) * NB;
-  const int cnt = min(NB, NH - k0);
-  const int w = 2 * a.radius + 1;
-  constexpr size_t ZS = (size_t)N * NH;  // elements per z step of the spectrum and weight
-  const int team = threadIdx.x / P, lane = threadIdx.x % P;
-  const int kl = team;  // consecutive columns for the teams of a warp
-  const int kx = k0 + kl;
+  const int ky = blockIdx.x, w = 2 * a.radius + 1;
+  const int col = threadIdx.x % TP, jt = threadIdx.x / TP;
+  const int kx = col == 0 ? N / 2 : col - 1;
+  const bool in = threadIdx.x < TP * JB, line = in && col < NH;  // whole warps' remainder, pad columns
   const double hw = (kx == 0 || 2 * kx == N) ? 1.0 : 2.0;
-
-  if (threadIdx.x == 0) mbar_init(&bar, 1);
+  constexpr size_t ZS = (size_t)N * NH;  // elements per z step of the spectrum and weight
+  const size_t at = (size_t)ky * NH + (line ? kx : 0);
+  // r < 8: of the last stage's R2 outputs only the first (z = m) and the last (z = m - 8) can lie in
+  // the window
+  const bool narrow = a.radius < 8;
   load_twiddles<N>(s_tw, g_tw);
-  __syncthreads();  // the barrier is initialised before anyone polls it
-  int loaded = -1;  // particle whose spectrum and weight rows are in shared memory
-  // one evaluation; returns false when its copy timed out (the CTA then leaves)
-  auto one = [&](const int k) -> bool {
+  int loaded = -1;  // particle whose spectrum and weight are in the registers (ONE)
+  float2 qr[8];
+  float wr[8];
+#pragma unroll 1
+  for (int k = 0; k < ne; ++k) {
     const int e = e_first + k;
     const EvalItem it = a.items[e];
     const DevParticle& pt = a.parts[it.particle];
     // weights on the rotated reference (BH_multi_xcf_Translational_2.m:35-38): the particle's
-    // wdgMask and the reference's bandpass wref; the first present one is copied, a second folded in
+    // wdgMask and the reference's bandpass wref
     const float* __restrict__ wref = a.refs[pt.ref].wref;
     const float* __restrict__ w1 = pt.wedge ? pt.wedge : wref;
     const float* __restrict__ w2 = pt.wedge ? wref : nullptr;
-    const float2* qrow = pt.spec + (size_t)ky * NH + k0;
-    const float* wrow = w1 ? w1 + (size_t)ky * NH + k0 : nullptr;
-    const bool piece_q = ((uintptr_t)pt.spec & 15) == 0;
-    const bool piece_w = C::PREF_W && w1 && ((uintptr_t)w1 & 15) == 0;
-    // row offsets (elements) from the 16-byte boundary below each row start, 16-byte pieces per row
-    const int offq = piece_q ? (int)(((uintptr_t)qrow & 15) >> 3) : 0;
-    const int offw = piece_w ? (int)(((uintptr_t)wrow & 15) >> 2) : 0;
-    const bool reload = it.particle != loaded;  // the same for the whole CTA
-    if (k > 0) __syncthreads();  // the previous evaluation is done with the tile (and the rows)
-    if (threadIdx.x == 0) {
-      if (k > 0) fence_proxy_async_shared();
-      mbar_arrive_expect_tx(&bar, SLAB_BYTES + a.phantom_tx);
-      bulk_copy_g2s(tile, a.s1 + (size_t)e * C::S1_EVAL + (size_t)blockIdx.x * C::PY * TP, SLAB_BYTES, &bar);
-    }
-    if (reload) {
-      const int pq = ((offq + cnt) * 8 + 15) >> 4;
-      const int pw = ((offw + cnt) * 4 + 15) >> 4;
-      if (piece_q) {
-        const char* src = reinterpret_cast<const char*>(qrow - offq);
-        for (int i = threadIdx.x; i < N * pq; i += NT) {
-          const int z = i / pq, c = i % pq;
-          cp_async16(reinterpret_cast<char*>(s_q + (size_t)z * QP) + 16 * c, src + z * ZS * sizeof(float2) + 16 * c);
-        }
-      } else {
-        for (int i = threadIdx.x; i < N * NB; i += NT)
-          if (i % NB < cnt) cp_async8(s_q + (i / NB) * QP + i % NB, qrow + (i / NB) * ZS + i % NB);
-      }
-      if (piece_w) {
-        const char* src = reinterpret_cast<const char*>(wrow - offw);
-        for (int i = threadIdx.x; i < N * pw; i += NT) {
-          const int z = i / pw, c = i % pw;
-          cp_async16(reinterpret_cast<char*>(s_w + (size_t)z * WP) + 16 * c, src + z * ZS * sizeof(float) + 16 * c);
-        }
-      } else if (C::PREF_W && w1) {
-        for (int i = threadIdx.x; i < N * NB; i += NT)
-          if (i % NB < cnt) cp_async4(s_w + (i / NB) * WP + i % NB, wrow + (i / NB) * ZS + i % NB);
-      }
-      cp_async_commit();
-      cp_async_wait<0>();
-    }
-    // the next barrier also publishes the cp.async pieces; the whole CTA takes the same branch
-    const bool arrived = mbar_wait(&bar, (unsigned)(k & 1), a.wait_cycles);
-    if (__syncthreads_or(!arrived)) {
-      // the copy did not complete in time: report, give it a second bounded wait, and leave
-      if (threadIdx.x == 0 && a.status) atomicOr(a.status, kStatusWaitTimeout);
-      mbar_wait(&bar, (unsigned)(k & 1), a.wait_cycles);
-      return false;
-    }
-    if (reload) {
-      if (C::PREF_W && w2) {
-        for (int i = threadIdx.x; i < N * NB; i += NT)
-          if (i % NB < cnt)
-            s_w[(i / NB) * WP + offw + i % NB] *= __ldg(w2 + (size_t)(i / NB) * ZS + (size_t)ky * NH + k0 + i % NB);
-        __syncthreads();
-      }
-      loaded = it.particle;
-    }
-
+    const float2* __restrict__ spec = pt.spec;
     const bool weighted = w1 != nullptr;
-    // E_R: each lane's |.|^2 over its elements of the line (8 to 16) in FP32, the lanes' partial
-    // sums then accumulated in FP64 (block_sum and the evaluation's atomicAdd)
-    float ef = 0.f;
-    {
-      const float2* sq = s_q + offq + kl;
-      const float* sw = s_w + offw + kl;
-      fft_line_fwd_mul_inv<N, P, 1>(tile + kl, TP, lane, s_tw, kl < cnt, [&](int z, float2 rr) {
-        const bool origin = z == 0 && ky == 0 && kx == 0;
-        if (weighted) {
-          float wv;
-          if constexpr (C::PREF_W) {
-            wv = sw[z * WP];
-          } else {  // read when the product is formed (128^3: no weight slab, three CTAs per SM)
-            const size_t gi = (size_t)z * ZS + (size_t)ky * NH + kx;
-            wv = __ldg(w1 + gi);
-            if (w2) wv *= __ldg(w2 + gi);
+    // spectrum and weight of butterfly k1 (kz = k1 + R2 k2)
+    auto fetch = [&](int k1) {
+#pragma unroll
+      for (int k2 = 0; k2 < 8; ++k2) {
+        const size_t i = (size_t)(k1 + R2 * k2) * ZS + at;
+        qr[k2] = __ldg(spec + i);
+        wr[k2] = w1 ? __ldg(w1 + i) : 1.f;
+        if (w2) wr[k2] *= __ldg(w2 + i);
+      }
+    };
+    __syncthreads();  // the previous evaluation is done with the buffer (and the twiddles are there)
+    const float2* s1 = a.s1 + (size_t)e * C::S1_EVAL + (size_t)ky * N * TP + col;
+    // first stage, from global memory: z = j + 8 r
+    if (in) {
+#pragma unroll 1
+      for (int j = jt; j < 8; j += JB) {
+        float2 v[R2];
+#pragma unroll
+        for (int r = 0; r < R2; ++r) v[r] = __ldcs(s1 + (size_t)(j + 8 * r) * TP);
+        Dft<R2, -1>::run(v);
+#pragma unroll
+        for (int k1 = 0; k1 < R2; ++k1) buf[k1 * ZA + j * TP + col] = v[k1];
+      }
+    }
+    if (line && (!ONE || it.particle != loaded)) fetch(jt);
+    loaded = it.particle;
+    __syncthreads();
+    // second stage, product, first inverse stage: kz = k1 + R2 k2 in registers
+    float ef = 0.f;  // |.|^2 of this thread's elements; the threads' sums are added in FP64
+    if (line) {
+#pragma unroll 1
+      for (int k1 = jt; k1 < R2; k1 += JB) {
+        float2* lp = buf + k1 * ZA + col;
+        float2 v[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[j] = lp[j * TP];
+#pragma unroll
+        for (int j = 1; j < 8; ++j) v[j] = cmul(v[j], s_tw[j * k1]);
+        Dft<8, -1>::run(v);
+#pragma unroll
+        for (int k2 = 0; k2 < 8; ++k2) {
+          const bool origin = k1 + R2 * k2 + ky + kx == 0;
+          float2 r = v[k2];
+          if (weighted) {
+            r.x *= wr[k2];
+            r.y *= wr[k2];
+            if (!origin) ef = fmaf(r.x, r.x, fmaf(r.y, r.y, ef));
           }
-          rr.x *= wv;
-          rr.y *= wv;
-          if (!origin) ef = fmaf(rr.x, rr.x, fmaf(rr.y, rr.y, ef));
+          const float2 x = cmulc(qr[k2], r);
+          v[k2] = origin ? make_float2(0.f, 0.f) : x;
         }
-        const float2 x = cmulc(sq[z * QP], rr);
-        return origin ? make_float2(0.f, 0.f) : x;
-      });
+        if (!ONE && k1 + JB < R2) fetch(k1 + JB);
+        Dft<8, 1>::run(v);
+#pragma unroll
+        for (int m = 1; m < 8; ++m) v[m] = cmulc(v[m], s_tw[m * k1]);
+#pragma unroll
+        for (int m = 0; m < 8; ++m) lp[m * TP] = v[m];
+      }
     }
     if (weighted) {
-      double t = block_sum(hw * (double)ef, red);
+      const double t = block_sum(line ? hw * (double)ef : 0.0, red);  // (synchronises)
       if (threadIdx.x == 0) atomicAdd(&a.stats[e].energy_spec, t);
+    } else {
+      __syncthreads();
     }
-    __syncthreads();
-    float2* dst = a.s2 + (size_t)e * w * C::S2_PLANE + (size_t)lpos<1>(ky) * C::PC + k0;
-    for (int i = threadIdx.x; i < w * NB; i += NT) {
-      const int j = i / NB, c = i % NB;
-      if (c >= cnt) continue;
-      const int z = (j - a.radius + N) % N;
-      dst[(size_t)j * C::S2_PLANE + c] = tile[lpos<1>(z) * TP + c];
+    // last inverse stage: z = m + 8 l, the planes |sz| <= r to S2
+    if (line) {
+      float2* dst = a.s2 + (size_t)e * w * C::S2_PLANE + (size_t)lpos<1>(ky) * C::PC + kx;
+#pragma unroll 1
+      for (int m = jt; m < 8; m += JB) {
+        float2 v[R2];
+#pragma unroll
+        for (int k1 = 0; k1 < R2; ++k1) v[k1] = buf[k1 * ZA + m * TP + col];
+        if (narrow) {
+          float2 first, last;
+          idft_ends<R2>(v, s_tw, first, last);
+          if (m <= a.radius) dst[(size_t)(m + a.radius) * C::S2_PLANE] = first;
+          if (8 - m <= a.radius) dst[(size_t)(m - 8 + a.radius) * C::S2_PLANE] = last;
+        } else {
+          Dft<R2, 1>::run(v);
+#pragma unroll
+          for (int l = 0; l < R2; ++l) {
+            const int z = m + 8 * l, sz = z < N / 2 ? z : z - N;
+            if (abs(sz) <= a.radius) dst[(size_t)(sz + a.radius) * C::S2_PLANE] = v[l];
+          }
+        }
+      }
     }
-    return true;
-  };
-  // straight-line calls (a rolled loop over evaluations let the compiler hoist the transforms'
-  // addressing out of it and spill)
-  static_assert(C::EVALS_B == 1 || C::EVALS_B == 2 || C::EVALS_B == 4, "1, 2 or 4 evaluations per CTA");
-  if (!one(0)) return;
-  if constexpr (C::EVALS_B > 1) {
-    if (ne < 2 || !one(1)) return;
   }
-  if constexpr (C::EVALS_B > 2) {
-    if (ne < 3 || !one(2)) return;
-    if (ne < 4) return;
-    one(3);
-  }
-}
-
-// 64^3: four resident 288-thread CTAs per SM asked of the compiler
-template <int N>
-__global__ void __launch_bounds__(SearchCfg<N>::NT_B, N <= 64 ? 4 : 0) k_search_z_mul(const SearchChunkArgs a,
-                                                                      const float2* __restrict__ g_tw) {
-  z_mul_bulk<N>(a, g_tw);
 }
 
 // ------------------------------------------------------------------ pass C

@@ -115,7 +115,7 @@ __global__ void k_noalloc_outputs(const NoallocResult* __restrict__ res, int n_o
 template <int N, typename T>
 emc_status set_attrs_noalloc() {
   using C = SearchCfg<N>;
-  EMC_CUDA(cudaFuncSetAttribute(k_search_fwd_xy<N, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM_A));
+  EMC_CUDA(cudaFuncSetAttribute(k_search_fwd_xy<N, T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM_A));
   EMC_CUDA(cudaFuncSetAttribute(k_search_z_mul<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM_B));
   EMC_CUDA(cudaFuncSetAttribute(k_search_inv_peak<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM_C));
   return EMC_OK;
@@ -165,8 +165,9 @@ emc_status run_chunks(const SearchChunkArgs& proto, int n_orient, int chunk, con
     a.n_items = std::min(chunk, n_orient - off);
     EMC_CUDA(cudaMemsetAsync(a.stats, 0, sizeof(EvalStats) * a.n_items, st));
     EMC_CUDA(cudaMemsetAsync(a.keys, 0, sizeof(unsigned long long) * a.n_items, st));
-    k_search_fwd_xy<N, float><<<dim3(N / C::G, a.n_items), C::NT_A, C::SMEM_A, st>>>(a, tw);
-    k_search_z_mul<N><<<dim3(C::GRID_BX, (a.n_items + C::EVALS_B - 1) / C::EVALS_B), C::NT_B, C::SMEM_B, st>>>(a, tw);
+    a.planes = 1;
+    k_search_fwd_xy<N, float, false><<<dim3(N, a.n_items), C::NT_A, C::SMEM_A, st>>>(a, tw);
+    k_search_z_mul<N><<<dim3(N, (a.n_items + C::EVALS_B - 1) / C::EVALS_B), C::NT_B, C::SMEM_B, st>>>(a, tw);
     k_search_inv_peak<N><<<dim3(w, a.n_items), C::NT_BC, C::SMEM_C, st>>>(a, tw);
     k_noalloc_decode<<<(a.n_items + 127) / 128, 128, 0, st>>>(a, N, res, best);
     EMC_LAUNCH_CHECK();
@@ -215,7 +216,7 @@ emc_status emc_search_plain_noalloc(const float* d_ref, const float* d_mask, int
   pt.box = n;
   pt.orient_begin = 0;
   pt.eval_base = 0;
-  DevRef rf{d_ref, d_mask, nullptr, n, EMC_DTYPE_F32};
+  DevRef rf{d_ref, d_mask, nullptr, n, EMC_DTYPE_F32, nullptr, nullptr, nullptr, nullptr};
   memcpy(host.data(), &pt, sizeof(pt));
   memcpy(host.data() + 256, &rf, sizeof(rf));
   double* dmat = reinterpret_cast<double*>(host.data() + (dm - hdr));
