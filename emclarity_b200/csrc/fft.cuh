@@ -595,6 +595,44 @@ __device__ __forceinline__ void fft_line_fwd_mul_inv(float2* buf, int stride, in
   InverseStagesReversed<L, P, PAD, LAST - 1, RL>::run(buf, stride, lane, tw, active);
 }
 
+// ---------------------------------------------------------------- lines across lanes
+// Mixed-radix stages for kernels whose neighbouring threads hold neighbouring lines: a thread has one
+// butterfly of its own line at a time, so accesses are consecutive in the lines whatever the strides, and
+// the stages work in place.  With M_s = L / (R_0 .. R_s), element n = sum r_s M_s starts at position n;
+// stage s replaces digit r_s (stride M_s) by the output digit k_s, so that X(k_0 + R_0 k_1 + ..) ends at
+// position sum k_s M_s, and the inverse over the same radices in reverse order ends in natural order.
+// The butterflies, twiddles and their order are those of the Stockham stages above: same bits.
+__host__ __device__ constexpr int digit_stride(int L, int s) { return L / radix_product(L, s + 1); }
+// Output index k_0 + R_0 k_1 + .. held by the leading digits `hi` (k_0 most significant) of a position.
+template <int L, int S>
+__device__ __forceinline__ int digit_index(int hi) {
+  if constexpr (S == 0) {
+    return 0;
+  } else if constexpr (S == 1) {
+    return hi;
+  } else {
+    constexpr int R = radix_of(L, S - 1);
+    return digit_index<L, S - 1>(hi / R) + radix_product(L, S - 1) * (hi % R);
+  }
+}
+// Butterfly b of forward or (same radices, same order) inverse stage S: its first position and its
+// index among the outputs formed so far.
+template <int L, int S>
+struct InPlace {
+  static constexpr int R = radix_of(L, S), M = digit_stride(L, S), NS = radix_product(L, S), NB = L / R;
+  static __device__ __forceinline__ int base(int b) { return (b / M) * (R * M) + b % M; }
+  static __device__ __forceinline__ int index(int b) { return digit_index<L, S>(b / M); }
+  // twiddles of a loaded butterfly, then its transform
+  template <int SIGN>
+  static __device__ __forceinline__ void run(float2 (&v)[R], int k, const float2* tw) {
+    if constexpr (NS > 1) {
+#pragma unroll
+      for (int r = 1; r < R; ++r) v[r] = cmul(v[r], twiddle<SIGN>(tw, r * k * (L / (NS * R))));
+    }
+    Dft<R, SIGN>::run(v);
+  }
+};
+
 // Loads the length-L twiddle table into shared memory (cooperatively, whole block).
 template <int L>
 __device__ __forceinline__ void load_twiddles(float2* s_tw, const float2* g_tw) {

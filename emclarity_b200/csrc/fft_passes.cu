@@ -46,25 +46,19 @@ static emc_status cols_t(const float2* in, float2* out, long stride, long inner,
   using C = ColsCfg<L>;
   const float2* tw = device_twiddles(L);
   if (!tw) return EMC_E_CUDA;
-  auto kern = k_cols<L, SIGN, C::P, C::T>;
-  // CTAs per SM, per device: the first launch on a device queries it; threads that race there both
-  // store the same value
-  static std::atomic<int> resident[64];
+  auto kern = k_cols<L, SIGN>;
+  // shared-memory opt-in, per device: threads that race on a device's first launch both make it
+  static std::atomic<bool> ready[64];
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 64) return EMC_E_CUDA;
-  int res = resident[dev].load(std::memory_order_acquire);
-  if (!res) {
-    if (C::smem > 48 * 1024)
-      EMC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::smem));
-    int nb = 0;
-    EMC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kern, C::P * C::T, C::smem));
-    res = std::max(nb, 1);
-    resident[dev].store(res, std::memory_order_release);
+  if (C::smem > 48 * 1024 && !ready[dev].load(std::memory_order_acquire)) {
+    EMC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::smem));
+    ready[dev].store(true, std::memory_order_release);
   }
-  const long units = (inner + C::T - 1) / C::T * outer;
-  const long ctas = std::min<long>(units, (long)res * device_sm_count());
-  kern<<<(unsigned)ctas, C::P * C::T, C::smem, st>>>(in, out, stride, inner, outer, outer_pitch, tw);
+  const long lines = inner * outer;
+  kern<<<(unsigned)((lines + C::T - 1) / C::T), C::T * C::J, C::smem, st>>>(in, out, stride, inner, lines, outer_pitch,
+                                                                           tw);
   EMC_LAUNCH_CHECK();
   return EMC_OK;
 }

@@ -106,68 +106,93 @@ __global__ void __launch_bounds__(256) k_rows_c2r(const float2* __restrict__ in,
 
 // ----------------------------------------------------------------- strided columns
 // Complex lines along a strided axis: element n of line (o, i) lives at
-// base + o*outer_pitch + i + n*stride, for i in [0, inner), o in [0, outer).
-// A unit of work is a tile of T consecutive i of one o; in == out is allowed (units are disjoint).
-// Persistent CTAs walk the units with a stride of gridDim.x and double-buffer them in shared
-// memory: the cp.async copies of the next tile are in flight while the current tile is
-// transformed and written back, so the loads of a one-CTA-per-SM kernel overlap its FFT.
-template <int L, int SIGN, int P, int T>
-__global__ void __launch_bounds__(P * T) k_cols(const float2* __restrict__ in, float2* __restrict__ out,
-                                                long stride, long inner, long outer, long outer_pitch,
-                                                const float2* __restrict__ g_tw) {
-  extern __shared__ float2 smem[];
-  constexpr int TP = T + 1;
-  constexpr int PAD = line_pad(L);
-  constexpr int TILE = padded_len(L, PAD) * TP;  // element n of line t at lpos<PAD>(n) * TP + t
-  float2* s_tw = smem;
-  float2* tiles = smem + L;  // [2][TILE]
-  load_twiddles<L>(s_tw, g_tw);
-  const long ntile = (inner + T - 1) / T;
-  const long units = ntile * outer;
-  constexpr int NT = P * T;
-  const int team = threadIdx.x / P, lane = threadIdx.x % P;
-  auto issue = [&](long u, float2* tile) {
-    const long o = u / ntile, i0 = (u % ntile) * T;
-    const float2* src = in + o * outer_pitch + i0;
-#pragma unroll 4
-    for (int idx = threadIdx.x; idx < L * T; idx += NT) {
-      const int n = idx / T, t = idx % T;
-      if (i0 + t < inner) cp_async8(tile + lpos<PAD>(n) * TP + t, src + (long)n * stride + t);
-    }
-    cp_async_commit();
-  };
-  long u = blockIdx.x;
-  if (u < units) issue(u, tiles);
-  int cur = 0;
-  for (; u < units; u += gridDim.x) {
-    const long un = u + gridDim.x;
-    if (un < units) {
-      issue(un, tiles + (cur ^ 1) * TILE);
-      cp_async_wait<1>();
+// base + o*outer_pitch + i + n*stride, for i in [0, inner), o in [0, outer); in == out is allowed.
+// A CTA transforms T consecutive lines (of the flattened (o, i), so that an inner extent that is no
+// multiple of T leaves no partial tiles) with J threads each, threads of a half-warp on consecutive
+// lines: the first stage takes its inputs from global memory, the last one stores its outputs there,
+// and only the exchanges between stages cross shared memory, in place and without bank conflicts
+// (twice per exchange; a tile copied in and out around teams that transform a line each crossed it
+// eight times at 512 points).  Several CTAs per SM overlap one's loads with the others' stages.
+template <int L>
+struct ColsCfg {
+  static constexpr int T = L <= 128 ? 32 : 16;
+  static constexpr int MOST = 512 / T;
+  // Threads per line: the count up to MOST whose rounds waste least over all stages, the largest such
+  // (an even count, so that T J is a multiple of 32).
+  static constexpr int padded_work(int J, int s = 0) {
+    return radix_of(L, s) <= 1 ? 0
+                               : (L / radix_of(L, s) + J - 1) / J * J * radix_of(L, s) + padded_work(J, s + 1);
+  }
+  static constexpr int best(int J, int found) {
+    return J > MOST || J > 2 * min_butterflies(L) ? found
+           : best(J + 2, padded_work(J) * 20 <= padded_work(found) * 21 ? J : found);
+  }
+  static constexpr int J = best(MOST / 4 + MOST / 4 % 2 > 2 ? MOST / 4 + MOST / 4 % 2 : 2,
+                                MOST / 4 + MOST / 4 % 2 > 2 ? MOST / 4 + MOST / 4 % 2 : 2);
+  static constexpr size_t smem = sizeof(float2) * (L + (size_t)L * T);
+  static constexpr int by_smem = (int)((220 * 1024) / (smem + 1024));
+  static constexpr int by_regs = 1024 / (T * J) > 1 ? 1024 / (T * J) : 1;  // 64 registers a thread
+  static constexpr int min_blocks = by_smem < by_regs ? by_smem : by_regs;
+};
+
+// One stage of a tile's lines.  ld(n) / st(k, v): global element access of this thread's line.
+template <int L, int SIGN, int T, int J, int S, class Ld, class St>
+__device__ __forceinline__ void cols_stage(float2* line, int jt, bool active, const float2* tw, const Ld& ld,
+                                           const St& st) {
+  using I = InPlace<L, S>;
+  constexpr bool FIRST = S == 0, LAST = S == n_stages(L) - 1;
+#pragma unroll(FIRST ? 2 : 1)
+  for (int b = jt; b < I::NB; b += J) {
+    const int base = I::base(b), k = I::index(b);
+    float2 v[I::R];
+    if (FIRST) {
+#pragma unroll
+      for (int r = 0; r < I::R; ++r) v[r] = active ? ld(base + r * I::M) : make_float2(0.f, 0.f);
     } else {
-      cp_async_wait<0>();
+#pragma unroll
+      for (int r = 0; r < I::R; ++r) v[r] = line[(base + r * I::M) * T];
     }
-    __syncthreads();  // tile `cur` (and the twiddles) visible to every thread
-    float2* tile = tiles + cur * TILE;
-    const long o = u / ntile, i0 = (u % ntile) * T;
-    fft_line<L, SIGN, P, PAD>(tile + team, TP, lane, s_tw, i0 + team < inner);
+    I::template run<SIGN>(v, k, tw);
+    if (LAST) {
+      if (active) {
+#pragma unroll
+        for (int r = 0; r < I::R; ++r) st(k + I::NS * r, v[r]);
+      }
+    } else {
+#pragma unroll
+      for (int r = 0; r < I::R; ++r) line[(base + r * I::M) * T] = v[r];
+    }
+  }
+  if constexpr (!LAST) {
     __syncthreads();
-    float2* dst = out + o * outer_pitch + i0;
-    for (int idx = threadIdx.x; idx < L * T; idx += NT) {
-      const int n = idx / T, t = idx % T;
-      if (i0 + t < inner) dst[(long)n * stride + t] = tile[lpos<PAD>(n) * TP + t];
-    }
-    __syncthreads();  // tile `cur` has been read; the next iteration's copies land in it
-    cur ^= 1;
+    cols_stage<L, SIGN, T, J, S + 1>(line, jt, active, tw, ld, st);
   }
 }
 
-template <int L>
-struct ColsCfg {
-  static constexpr int P = team_size(L);
-  static constexpr int T = (512 / P) < 32 ? (512 / P) : 32;
-  static constexpr size_t smem = sizeof(float2) * (L + 2 * (size_t)padded_len(L, line_pad(L)) * (T + 1));
-};
+template <int L, int SIGN>
+__global__ void __launch_bounds__(ColsCfg<L>::T * ColsCfg<L>::J, ColsCfg<L>::min_blocks) k_cols(
+    const float2* __restrict__ in, float2* __restrict__ out, long stride, long inner, long lines, long outer_pitch,
+    const float2* __restrict__ g_tw) {
+  using C = ColsCfg<L>;
+  extern __shared__ float2 smem[];
+  float2* s_tw = smem;
+  load_twiddles<L>(s_tw, g_tw);
+  const int t = threadIdx.x % C::T, jt = threadIdx.x / C::T;
+  const long c0 = (long)blockIdx.x * C::T;
+  long o = c0 / inner, i = c0 - o * inner + t;  // the division is the same for the whole CTA
+  while (i >= inner) {
+    i -= inner;
+    ++o;
+  }
+  const bool active = c0 + t < lines;
+  const long at = o * outer_pitch + i;
+  const float2* src = in + at;
+  float2* dst = out + at;
+  if constexpr (n_stages(L) > 1) __syncthreads();  // the twiddles
+  cols_stage<L, SIGN, C::T, C::J, 0>(
+      smem + L + t, jt, active, s_tw, [&](int n) { return src[(long)n * stride]; },
+      [&](int k, float2 v) { dst[(long)k * stride] = v; });
+}
 
 // Host launchers (defined in fft_passes.cu); return EMC_OK or an error status.
 emc_status launch_rows_r2c(int L, const float* in, long in_pitch, float2* out, long out_pitch, long nrows,

@@ -99,74 +99,127 @@ __global__ void __launch_bounds__(256) k_ts_rows(const float* __restrict__ tmpl,
   }
 }
 
-// Per tile of TT consecutive (ky, kx) z-lines: G = FFT_z of the t planes at z = pl[2].. (zeros
+// Per tile of T consecutive (ky, kx) z-lines: G = FFT_z of the t planes at z = pl[2].. (zeros
 // elsewhere), X = T .* conj(G), inverse FFT_z into s.  stats[0] += sum over the full spectrum of
-// |X|^2 (Hermitian weights), stats[1] = X(0).  The product and statistics are formed in registers
-// between the two transforms (fft_line_fwd_mul_inv).
-// Resident CTAs per SM asked of the compiler: 20 warps' worth when a lane holds at most 16 complex
-// values per stage (the register cap then leaves room for them), else no constraint.
-constexpr int zfused_min_blocks(int L, int P, int TT) {
-  return stage_values(L, P) <= 16 && 640 / (P * TT) > 1 ? 640 / (P * TT) : 1;
+// |X|^2 (Hermitian weights), stats[1] = X(0).  The forward transform's last stage leaves a butterfly's
+// outputs k' + (L / RL) r in registers, the inputs of the inverse transform's first stage when it takes
+// the radices in reverse order: the product and the statistics are formed there.  Neighbouring threads
+// hold neighbouring lines (see k_cols): inputs come from and results go to global memory directly.
+template <int L>
+struct ZfusedCfg {
+  static constexpr int P = team_size(L);          // threads per line (the statistics' partial sums)
+  static constexpr int T = P >= 16 ? 16 : P >= 8 ? 32 : 256 / P;
+  static constexpr size_t smem = sizeof(float2) * (L + (size_t)L * T);
+  static constexpr int by_smem = (int)((220 * 1024) / (smem + 1024));
+  static constexpr int by_regs = 1024 / (T * P) > 1 ? 1024 / (T * P) : 1;
+  static constexpr int min_blocks = by_smem < 1 ? 1 : by_smem < by_regs ? by_smem : by_regs;
+};
+
+// Forward stages S .. LAST - 1, then (S == LAST) the product and the inverse's first stage.
+template <int L, int T, int P, int S, class Ld, class Mul>
+__device__ __forceinline__ void zfused_forward(float2* line, int jt, const float2* tw, const Ld& ld, const Mul& mul) {
+  using I = InPlace<L, S>;
+  constexpr bool LAST = S == n_stages(L) - 1;
+#pragma unroll 1
+  for (int b = jt; b < I::NB; b += P) {
+    const int base = I::base(b), k = I::index(b);
+    float2 v[I::R];
+#pragma unroll
+    for (int r = 0; r < I::R; ++r) v[r] = S == 0 ? ld(base + r * I::M) : line[(base + r * I::M) * T];
+    I::template run<-1>(v, k, tw);
+    if constexpr (LAST) {
+      mul(k, v);  // element k + NS r in v[r]
+      Dft<I::R, 1>::run(v);
+    }
+#pragma unroll
+    for (int r = 0; r < I::R; ++r) line[(base + r * I::M) * T] = v[r];
+  }
+  __syncthreads();
+  if constexpr (!LAST) zfused_forward<L, T, P, S + 1>(line, jt, tw, ld, mul);
 }
 
-template <int L, int P, int TT>
-__global__ void __launch_bounds__(P * TT, zfused_min_blocks(L, P, TT)) k_ts_zfused(const float2* __restrict__ gt, const float2* __restrict__ T,
-                                                      float2* __restrict__ s, const TsGeom g,
-                                                      double* __restrict__ stats, const float2* __restrict__ g_tw) {
+// Inverse stages over the forward radices S .. 0 (NS: product of the radices already taken); the
+// outputs formed so far are indexed by a position's trailing digits.
+template <int L, int T, int P, int S, int NS, class St>
+__device__ __forceinline__ void zfused_inverse(float2* line, int jt, const float2* tw, const St& st) {
+  constexpr int R = radix_of(L, S), M = digit_stride(L, S), NB = L / R;
+  static_assert(M == NS, "trailing digits");
+#pragma unroll 1
+  for (int b = jt; b < NB; b += P) {
+    const int k = b % M, base = (b / M) * (R * M) + k;
+    float2 v[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) v[r] = line[(base + r * M) * T];
+#pragma unroll
+    for (int r = 1; r < R; ++r) v[r] = cmul(v[r], twiddle<1>(tw, r * k * (L / (NS * R))));
+    Dft<R, 1>::run(v);
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      if constexpr (S == 0) st(k + M * r, v[r]);
+      else line[(base + r * M) * T] = v[r];
+    }
+  }
+  if constexpr (S > 0) {
+    __syncthreads();
+    zfused_inverse<L, T, P, S - 1, NS * R>(line, jt, tw, st);
+  }
+}
+
+template <int L>
+__global__ void __launch_bounds__(ZfusedCfg<L>::T * ZfusedCfg<L>::P, ZfusedCfg<L>::min_blocks) k_ts_zfused(
+    const float2* __restrict__ gt, const float2* __restrict__ T, float2* __restrict__ s, const TsGeom g,
+    double* __restrict__ stats, const float2* __restrict__ g_tw) {
+  using C = ZfusedCfg<L>;
+  constexpr int LAST = n_stages(L) - 1, RL = radix_of(L, LAST), NT = C::T * C::P;
+  static_assert(NT % 32 == 0, "the statistics reduction needs whole warps");
   extern __shared__ float2 smem[];
-  constexpr int TP = TT + 1;
-  constexpr int PAD = line_pad(L);
-  float2* s_tw = smem;
-  float2* tile = smem + L;                                // [padded L][TP], element n of line t at lpos<PAD>(n) * TP + t
-  float2* s_t = tile + (size_t)padded_len(L, PAD) * TP;  // [L][TT], the tomogram spectrum of the tile's lines
-  static_assert((P * TT) % 32 == 0, "the statistics reduction needs whole warps");
   __shared__ double red[32];
+  float2* s_tw = smem;
   load_twiddles<L>(s_tw, g_tw);
-  const long inner = (long)g.ny * g.nxh, stride = inner;
-  const long i0 = (long)blockIdx.x * TT;
-  constexpr int NT = P * TT;
-  constexpr int IT = (L * TT + NT - 1) / NT;
-  // the tomogram spectrum of this tile, copied asynchronously while the template planes load
-#pragma unroll
-  for (int k = 0; k < IT; ++k) {
-    const int idx = threadIdx.x + k * NT;
-    const int n = idx / TT, t = idx % TT;
-    if (idx < L * TT && i0 + t < inner) cp_async8(s_t + idx, T + (long)n * stride + i0 + t);
-  }
-  cp_async_commit();
-  {
-    float2 v[IT];
-#pragma unroll
-    for (int k = 0; k < IT; ++k) {
-      const int idx = threadIdx.x + k * NT;
-      const int n = idx / TT, t = idx % TT;
-      const long i = i0 + t;
-      v[k] = make_float2(0.f, 0.f);
-      if (idx < L * TT && i < inner && n >= g.pl[2] && n < g.pl[2] + g.t) v[k] = gt[(long)(n - g.pl[2]) * stride + i];
-    }
-#pragma unroll
-    for (int k = 0; k < IT; ++k) {
-      const int idx = threadIdx.x + k * NT;
-      if (idx < L * TT) tile[lpos<PAD>(idx / TT) * TP + idx % TT] = v[k];
-    }
-  }
-  cp_async_wait<0>();
-  __syncthreads();
-  const int team = threadIdx.x / P, lane = threadIdx.x % P;
-  const long i = i0 + team;
-  const bool line_active = i < inner;
+  const int t = threadIdx.x % C::T, jt = threadIdx.x / C::T;
+  const long inner = (long)g.ny * g.nxh;
+  const long i = (long)blockIdx.x * C::T + t;
+  const bool active = i < inner;
+  const float2* gti = gt + i;
+  const float2* ti = T + i;
+  float2* si = s + i;
   const double hw = ((int)(i % g.nxh) == 0 || 2 * (int)(i % g.nxh) == g.nx) ? 1.0 : 2.0;
-  // forward z transform of the template planes, X = T .* conj(G) and its statistics in registers,
-  // inverse z transform (fft_line_fwd_mul_inv).  Each lane sums its elements' |X|^2 in FP32 (L / P
-  // of them), the lanes' sums are accumulated in FP64.
+  float2* line = smem + L + t;
+  __syncthreads();
+  // Each thread sums its elements' |X|^2 in FP32 (L / P of them), the threads' sums are accumulated in
+  // FP64.
   float ef = 0.f;
-  fft_line_fwd_mul_inv<L, P, PAD>(tile + team, TP, lane, s_tw, line_active, [&](int n, float2 gz) {
-    const float2 x = cmulc(s_t[n * TT + team], gz);
-    ef = fmaf(x.x, x.x, fmaf(x.y, x.y, ef));
-    if (i == 0 && n == 0) stats[1] = (double)x.x;
-    return x;
-  });
-  double e = hw * (double)ef;
+  zfused_forward<L, C::T, C::P, 0>(
+      line, jt, s_tw,
+      [&](int n) {
+        const int zt = n - g.pl[2];
+        return active && zt >= 0 && zt < g.t ? gti[(long)zt * inner] : make_float2(0.f, 0.f);
+      },
+      [&](int k, float2 (&v)[RL]) {
+        float2 tz[RL];
+#pragma unroll
+        for (int r = 0; r < RL; ++r)
+          tz[r] = active ? __ldg(ti + (long)(k + (L / RL) * r) * inner) : make_float2(0.f, 0.f);
+#pragma unroll
+        for (int r = 0; r < RL; ++r) {
+          const float2 x = cmulc(tz[r], v[r]);
+          ef = fmaf(x.x, x.x, fmaf(x.y, x.y, ef));
+          if (i == 0 && k + r == 0) stats[1] = (double)x.x;
+          v[r] = x;
+        }
+      });
+  auto store = [&](int n, float2 v) {
+    if (active) si[(long)n * inner] = v;
+  };
+  if constexpr (LAST > 0) {
+    zfused_inverse<L, C::T, C::P, LAST - 1, RL>(line, jt, s_tw, store);
+  } else {
+    // a single stage: its outputs are in the thread's own slots
+    for (int b = jt; b < L / RL; b += C::P)
+#pragma unroll
+      for (int r = 0; r < RL; ++r) store(r, line[r * C::T]);
+  }
+  double e = active ? hw * (double)ef : 0.0;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) e += __shfl_xor_sync(0xffffffffu, e, o);
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = e;
@@ -175,10 +228,6 @@ __global__ void __launch_bounds__(P * TT, zfused_min_blocks(L, P, TT)) k_ts_zfus
     double tot = 0.0;
     for (int w = 0; w < NT / 32; ++w) tot += red[w];
     atomicAdd(stats, tot);
-  }
-  for (int idx = threadIdx.x; idx < L * TT; idx += NT) {
-    const int n = idx / TT, t = idx % TT;
-    if (i0 + t < inner) s[(long)n * stride + i0 + t] = tile[lpos<PAD>(n) * TP + t];
   }
 }
 
@@ -357,24 +406,20 @@ static emc_status ts_rows_any(int L, const float* tmpl, const TsGeom& g, float2*
 template <int L>
 static emc_status launch_ts_zfused(const float2* gt, const float2* T, float2* s, const TsGeom& g, double* stats,
                                    cudaStream_t st) {
-  using C = ColsCfg<L>;
+  using C = ZfusedCfg<L>;
   const float2* tw = device_twiddles(L);
   if (!tw) return EMC_E_CUDA;
-  // Narrow tiles (8 lines, or one warp when the team is smaller than 4 lanes) keep several CTAs
-  // resident per SM, so one CTA's loads overlap another's transforms.
-  constexpr int TT = C::P >= 4 ? 8 : 32 / C::P;
-  auto kern = k_ts_zfused<L, C::P, TT>;
-  constexpr size_t smem = sizeof(float2) * (L + (size_t)padded_len(L, line_pad(L)) * (TT + 1) + (size_t)L * TT);
+  auto kern = k_ts_zfused<L>;
   static bool attr_set[64] = {false};
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 64) return EMC_E_CUDA;
-  if (smem > 48 * 1024 && !attr_set[dev]) {
-    EMC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (C::smem > 48 * 1024 && !attr_set[dev]) {
+    EMC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::smem));
     attr_set[dev] = true;
   }
   const long inner = (long)g.ny * g.nxh;
-  kern<<<(unsigned)((inner + TT - 1) / TT), C::P * TT, smem, st>>>(gt, T, s, g, stats, tw);
+  kern<<<(unsigned)((inner + C::T - 1) / C::T), C::T * C::P, C::smem, st>>>(gt, T, s, g, stats, tw);
   EMC_LAUNCH_CHECK();
   return EMC_OK;
 }
