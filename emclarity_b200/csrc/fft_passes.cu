@@ -118,6 +118,41 @@ emc_status fft3_r2c(const float* in, float2* out, int nx, int ny, int nz, int ba
   return EMC_OK;
 }
 
+template <int L>
+static emc_status cols_weighted_t(float2* q, int count, const float* wgt, const float* bp, double* energy,
+                                  cudaStream_t st) {
+  using C = ColsCfg<L>;
+  const float2* tw = device_twiddles(L);
+  if (!tw) return EMC_E_CUDA;
+  static std::atomic<bool> ready[64];
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev >= 64) return EMC_E_CUDA;
+  if (C::smem > 48 * 1024 && !ready[dev].load(std::memory_order_acquire)) {
+    EMC_CUDA(cudaFuncSetAttribute(k_cols_weighted<L>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::smem));
+    ready[dev].store(true, std::memory_order_release);
+  }
+  constexpr int INNER = L * (L / 2 + 1);
+  k_cols_weighted<L><<<dim3((INNER + C::T - 1) / C::T, count), C::T * C::J, C::smem, st>>>(q, wgt, bp, energy, tw);
+  EMC_LAUNCH_CHECK();
+  return EMC_OK;
+}
+
+emc_status weighted_spectra(const float* in, float2* out, int n, int count, const float* wgt, const float* bp,
+                            double* energy, cudaStream_t st) {
+  const long nxh = n / 2 + 1;
+  EMC_TRY(launch_rows_r2c(n, in, n, out, nxh, (long)n * n * count, st));
+  EMC_TRY(launch_cols(n, -1, out, out, nxh, nxh, (long)n * count, (long)n * nxh, st));
+  EMC_CUDA(cudaMemsetAsync(energy, 0, sizeof(double) * count, st));
+  switch (n) {
+#define X(L) case L: return cols_weighted_t<L>(out, count, wgt, bp, energy, st);
+    EMC_FOR_EACH_LENGTH(X)
+#undef X
+  }
+  set_error("FFT length %d not supported", n);
+  return EMC_E_UNSUPPORTED;
+}
+
 emc_status fft3_c2r(const float2* in, float* out, float2* scratch, int nx, int ny, int nz, int batch,
                     cudaStream_t st) {
   const long nxh = nx / 2 + 1;

@@ -194,6 +194,57 @@ __global__ void __launch_bounds__(ColsCfg<L>::T * ColsCfg<L>::J, ColsCfg<L>::min
       [&](int k, float2 v) { dst[(long)k * stride] = v; });
 }
 
+// The forward z transform of `count` n^3 half spectra in place, with the weighting that follows it in a
+// particle spectrum: q <- w b F, q(0) = 0, and the energies sum |q|^2 over the full spectra added in FP64
+// (wgt: one half spectrum per volume, bp: one shared, either may be null).  The last stage's outputs are
+// weighted in registers, so the spectra are not read and written once more.  Tiles stay inside a
+// volume (blockIdx.y).
+template <int L>
+__global__ void __launch_bounds__(ColsCfg<L>::T * ColsCfg<L>::J, ColsCfg<L>::min_blocks) k_cols_weighted(
+    float2* __restrict__ q, const float* __restrict__ wgt, const float* __restrict__ bp, double* __restrict__ energy,
+    const float2* __restrict__ g_tw) {
+  using C = ColsCfg<L>;
+  constexpr int NH = L / 2 + 1, INNER = NH * L;
+  constexpr int NT = C::T * C::J;
+  static_assert(NT % 32 == 0, "whole warps");
+  extern __shared__ float2 smem[];
+  __shared__ double red[32];
+  float2* s_tw = smem;
+  load_twiddles<L>(s_tw, g_tw);
+  const int t = threadIdx.x % C::T, jt = threadIdx.x / C::T;
+  const int i = blockIdx.x * C::T + t;
+  const bool active = i < INNER;
+  const int kx = i % NH;
+  const double hw = kx == 0 || 2 * kx == L ? 1.0 : 2.0;
+  float2* line = q + (long)blockIdx.y * L * INNER + i;
+  const float* wl = wgt ? wgt + (long)blockIdx.y * L * INNER + i : nullptr;
+  const float* bl = bp ? bp + i : nullptr;
+  double e = 0.0;
+  if constexpr (n_stages(L) > 1) __syncthreads();  // the twiddles
+  cols_stage<L, -1, C::T, C::J, 0>(
+      smem + L + t, jt, active, s_tw, [&](int n) { return line[(long)n * INNER]; },
+      [&](int k, float2 v) {
+        float f = 1.f;
+        if (wl) f *= __ldg(wl + (long)k * INNER);
+        if (bl) f *= __ldg(bl + (long)k * INNER);
+        if (i == 0 && k == 0) f = 0.f;
+        v.x *= f;
+        v.y *= f;
+        line[(long)k * INNER] = v;
+        e += (double)v.x * v.x + (double)v.y * v.y;
+      });
+  e *= hw;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) e += __shfl_xor_sync(0xffffffffu, e, o);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = e;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double tot = 0.0;
+    for (int w = 0; w < NT / 32; ++w) tot += red[w];
+    atomicAdd(energy + blockIdx.y, tot);
+  }
+}
+
 // Host launchers (defined in fft_passes.cu); return EMC_OK or an error status.
 emc_status launch_rows_r2c(int L, const float* in, long in_pitch, float2* out, long out_pitch, long nrows,
                            cudaStream_t st);
@@ -201,6 +252,11 @@ emc_status launch_rows_c2r(int L, const float2* in, long in_pitch, float* out, l
                            cudaStream_t st);
 emc_status launch_cols(int L, int sign, const float2* in, float2* out, long stride, long inner, long outer,
                        long outer_pitch, cudaStream_t st);
+
+// Particle spectra: the R2C transform of `count` n^3 volumes, weighted, and their energies (cleared here);
+// see k_cols_weighted.
+emc_status weighted_spectra(const float* in, float2* out, int n, int count, const float* wgt, const float* bp,
+                            double* energy, cudaStream_t st);
 
 // Full 3-D R2C / C2R over a batch of volumes (x fastest).  c2r uses `scratch`
 // ((nx/2+1)*ny*nz*batch float2) so that `in` is left untouched.

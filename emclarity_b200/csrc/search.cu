@@ -215,31 +215,6 @@ struct DevBuf {
   }
 };
 
-// Weights particle blockIdx.y of a batch (spectra, weights and energies advance by nhalf, nhalf and
-// 1 per particle; wgt_stride 0 shares one weight) and accumulates its energy.
-__global__ void k_particle_weight(float2* __restrict__ q, const float* __restrict__ wgt, const float* __restrict__ bp,
-                                  long nhalf, int nh, int n, double* __restrict__ energy, long wgt_stride = 0) {
-  __shared__ double red[32];
-  q += (long)blockIdx.y * nhalf;
-  if (wgt) wgt += (long)blockIdx.y * wgt_stride;
-  energy += blockIdx.y;
-  double e = 0.0;
-  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < nhalf; i += (long)gridDim.x * blockDim.x) {
-    float f = 1.f;
-    if (wgt) f *= wgt[i];
-    if (bp) f *= bp[i];
-    if (i == 0) f = 0.f;
-    float2 v = q[i];
-    v.x *= f;
-    v.y *= f;
-    q[i] = v;
-    const int kx = (int)(i % nh);
-    e += (kx == 0 || 2 * kx == n ? 1.0 : 2.0) * ((double)v.x * v.x + (double)v.y * v.y);
-  }
-  double t = block_sum(e, red);
-  if (threadIdx.x == 0) atomicAdd(energy, t);
-}
-
 }  // namespace emc
 
 // ===================================================================== C-ABI
@@ -1018,14 +993,8 @@ emc_status emc_particle_spectrum(int n, const float* d_particle, const float* d_
   EMC_CHECK_ARG(d_particle && d_spectrum_out && d_energy, "emc_particle_spectrum: null argument");
   EMC_CHECK_ARG(emc::fft_length_supported(n) && n >= 2, "emc_particle_spectrum: box %d not supported", n);
   cudaStream_t st = emc::as_stream(stream);
-  float2* q = reinterpret_cast<float2*>(d_spectrum_out);
-  EMC_TRY(emc::fft3_r2c(d_particle, q, n, n, n, 1, st));
-  EMC_CUDA(cudaMemsetAsync(d_energy, 0, sizeof(double), st));
-  const long nhalf = (long)(n / 2 + 1) * n * n;
-  const int blocks = (int)std::min<long>((nhalf + 255) / 256, 2L * emc::device_sm_count());
-  emc::k_particle_weight<<<blocks, 256, 0, st>>>(q, d_weight, d_bandpass, nhalf, n / 2 + 1, n, d_energy);
-  EMC_LAUNCH_CHECK();
-  return EMC_OK;
+  return emc::weighted_spectra(d_particle, reinterpret_cast<float2*>(d_spectrum_out), n, 1, d_weight, d_bandpass,
+                               d_energy, st);
 }
 
 emc_status emc_particle_spectra(int n, int count, const float* d_particles, const float* d_weights,
@@ -1034,15 +1003,8 @@ emc_status emc_particle_spectra(int n, int count, const float* d_particles, cons
   EMC_CHECK_ARG(emc::fft_length_supported(n) && n >= 2, "emc_particle_spectra: box %d not supported", n);
   EMC_CHECK_ARG(count <= 65535, "emc_particle_spectra: at most 65535 particles per call (got %d)", count);
   cudaStream_t st = emc::as_stream(stream);
-  float2* q = reinterpret_cast<float2*>(d_spectra_out);
-  EMC_TRY(emc::fft3_r2c(d_particles, q, n, n, n, count, st));
-  EMC_CUDA(cudaMemsetAsync(d_energies, 0, sizeof(double) * count, st));
-  const long nhalf = (long)(n / 2 + 1) * n * n;
-  const int bx = (int)std::max<long>(1, std::min<long>((nhalf + 255) / 256, (2L * emc::device_sm_count() + count - 1) / count));
-  emc::k_particle_weight<<<dim3(bx, count), 256, 0, st>>>(q, d_weights, d_bandpass, nhalf, n / 2 + 1, n, d_energies,
-                                                          nhalf);
-  EMC_LAUNCH_CHECK();
-  return EMC_OK;
+  return emc::weighted_spectra(d_particles, reinterpret_cast<float2*>(d_spectra_out), n, count, d_weights, d_bandpass,
+                               d_energies, st);
 }
 
 emc_status emc_particle_template(int n, const float* d_spectrum, float* d_h, void* stream) {
