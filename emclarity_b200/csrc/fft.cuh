@@ -399,20 +399,6 @@ template <int L, int SIGN, int P, int PAD, int S>
 struct StageChain<L, SIGN, P, PAD, S, L> {
   static __device__ __forceinline__ void run(float2*, int, int, const float2*, bool, const TwChain<L, P, S, L>*) {}
 };
-// Stages S .. LAST-1 only (NS = product of the radices before S).
-template <int L, int SIGN, int P, int PAD, int S, int NS, int LAST>
-struct ForwardMidStages {
-  static __device__ __forceinline__ void run(float2* buf, int stride, int lane, const float2* tw, bool active,
-                                             const TwChain<L, P, S, NS>* tc) {
-    if constexpr (S < LAST) {
-      constexpr int R = radix_of(L, S);
-      stockham_stage<L, R, NS, SIGN, P, PAD, S>(buf, stride, lane, tw, active, tc ? &tc->st : nullptr);
-      ForwardMidStages<L, SIGN, P, PAD, S + 1, NS * R, LAST>::run(buf, stride, lane, tw, active,
-                                                                 tc ? &tc->next : nullptr);
-    }
-  }
-};
-
 // First stage (NS = 1, no twiddles) with its inputs produced by ld(i) -- element i of the line
 // -- instead of loaded from the buffer, so a caller that builds the line (packing two real rows,
 // Hermitian extension) skips one shared-memory round trip.
@@ -456,144 +442,9 @@ __device__ __forceinline__ void fft_line_in(const Ld& ld, float2* buf, int strid
   StageChain<L, SIGN, P, PAD, 1, R0>::run(buf, stride, lane, tw, active, tc ? &tc->next : nullptr);
 }
 
-// Number of Stockham stages of a length-L plan and the product of the radices before stage s.
-__host__ __device__ constexpr int n_stages(int L, int s = 0);
-__host__ __device__ constexpr int radix_product(int L, int s);
-
-// The last Stockham stage of a length-L plan for teams of P lanes: radix RL, NSL = L / RL
-// butterflies (the product of the earlier radices), PER butterflies per lane.
-template <int L, int P>
-struct LastStage {
-  static constexpr int S = n_stages(L) - 1;
-  static constexpr int RL = radix_of(L, S);
-  static constexpr int NSL = L / RL;
-  static constexpr int PER = (NSL + P - 1) / P;
-};
-
-// Register twiddles of stage S of a chain (nullptr when the chain holds none for it).
-template <int S, int L, int P, int S0, int NS>
-__device__ __forceinline__ const StageTw<L, P, S, radix_product(L, S)>* stage_tw(const TwChain<L, P, S0, NS>* tc) {
-  if constexpr (S0 == S) {
-    return tc ? &tc->st : nullptr;
-  } else {
-    return stage_tw<S>(tc ? &tc->next : (const TwChain<L, P, S0 + 1, NS * radix_of(L, S0)>*)nullptr);
-  }
-}
-
-// FFT of a line whose elements come from ld(i), like fft_line_in, with the last stage left in
-// registers: on return v[b][r] holds element (lane + b P) + NSL r of the transform for every
-// butterfly lane + b P < NSL of an active lane (LastStage<L, P>); buf holds the earlier stages'
-// scratch.  The caller synchronises the team before buf is written again.
-template <int L, int SIGN, int P, int PAD, class Ld>
-__device__ __forceinline__ void fft_line_in_regs(const Ld& ld, float2* buf, int stride, int lane, const float2* tw,
-                                                 bool active, const LineTw<L, P>* tc,
-                                                 float2 (&v)[LastStage<L, P>::PER][LastStage<L, P>::RL]) {
-  using LS = LastStage<L, P>;
-  constexpr int R0 = radix_of(L, 0);
-  static_assert(LS::S >= 1, "at least two stages");
-  stockham_first_stage_in<L, R0, SIGN, P, PAD>(ld, buf, stride, lane, active);
-  if constexpr (LS::S > 1) {
-    // stages 1 .. S-1 in shared memory
-    ForwardMidStages<L, SIGN, P, PAD, 1, R0, LS::S>::run(buf, stride, lane, tw, active, tc ? &tc->next : nullptr);
-  }
-  const auto* cache = stage_tw<LS::S>(tc);
-#pragma unroll
-  for (int b = 0; b < LS::PER; ++b) {
-    const int j = lane + b * P;
-    if (active && (LS::PER * P == LS::NSL || j < LS::NSL)) {
-#pragma unroll
-      for (int r = 0; r < LS::RL; ++r) v[b][r] = buf[lpos<PAD>(j + r * LS::NSL) * stride];
-      if constexpr (StageTw<L, P, LS::S, LS::NSL>::kOn) {
-        if (cache) {
-#pragma unroll
-          for (int r = 1; r < LS::RL; ++r)
-            v[b][r] = SIGN < 0 ? cmul(v[b][r], cache->w[b][r - 1]) : cmulc(v[b][r], cache->w[b][r - 1]);
-        } else {
-#pragma unroll
-          for (int r = 1; r < LS::RL; ++r) v[b][r] = cmul(v[b][r], twiddle<SIGN>(tw, (r * j) % L));
-        }
-      } else {
-#pragma unroll
-        for (int r = 1; r < LS::RL; ++r) v[b][r] = cmul(v[b][r], twiddle<SIGN>(tw, (r * j) % L));
-      }
-      Dft<LS::RL, SIGN>::run(v[b]);
-    }
-  }
-}
-__host__ __device__ constexpr int n_stages(int L, int s) { return radix_of(L, s) <= 1 ? s : n_stages(L, s + 1); }
+// Number of stages of a length-L plan and the product of the radices before stage s.
+__host__ __device__ constexpr int n_stages(int L, int s = 0) { return radix_of(L, s) <= 1 ? s : n_stages(L, s + 1); }
 __host__ __device__ constexpr int radix_product(int L, int s) { return s == 0 ? 1 : radix_of(L, s - 1) * radix_product(L, s - 1); }
-
-// Forward stages S .. LAST-1 of a length-L line (NS = product of the radices before S).
-template <int L, int P, int PAD, int S, int LAST>
-struct ForwardStages {
-  static __device__ __forceinline__ void run(float2* buf, int stride, int lane, const float2* tw, bool active) {
-    if constexpr (S < LAST) {
-      stockham_stage<L, radix_of(L, S), radix_product(L, S), -1, P, PAD, S>(buf, stride, lane, tw, active, nullptr);
-      ForwardStages<L, P, PAD, S + 1, LAST>::run(buf, stride, lane, tw, active);
-    }
-  }
-};
-// Inverse stages with the forward radices taken in reverse order, from forward stage S down to 0
-// (NS = product of the radices already applied).  A mixed-radix transform may take its radices in
-// any order; this one starts with the forward plan's last radix.
-template <int L, int P, int PAD, int S, int NS>
-struct InverseStagesReversed {
-  static __device__ __forceinline__ void run(float2* buf, int stride, int lane, const float2* tw, bool active) {
-    if constexpr (S >= 0) {
-      stockham_stage<L, radix_of(L, S), NS, 1, P, PAD, S>(buf, stride, lane, tw, active, nullptr);
-      InverseStagesReversed<L, P, PAD, S - 1, NS * radix_of(L, S)>::run(buf, stride, lane, tw, active);
-    }
-  }
-};
-template <int L, int P, int PAD, int NS>
-struct InverseStagesReversed<L, P, PAD, -1, NS> {
-  static __device__ __forceinline__ void run(float2*, int, int, const float2*, bool) {}
-};
-
-// Forward transform, elementwise product, inverse transform of one line, with the product formed in
-// registers.  The forward transform's stages but the last run in shared memory; its last stage
-// (radix RL, NS = L / RL) leaves lane j of the team holding, for each of its butterflies
-// j' = j + b P, the elements z = j' + (L / RL) r -- the elements the inverse transform's first stage
-// needs when the inverse takes the radices in reverse order (radix RL first, NB = L / RL).  So
-// mul(z, X(z)) -> Y(z) is applied to those registers, the inverse's first stage runs on them and its
-// remaining stages in shared memory: two shared-memory passes over the line fewer than
-// fft_line(-1), a separate product and fft_line(+1).  Element i of the line lives at
-// buf[lpos<PAD>(i) * stride]; the result (unnormalised) is left there in natural order.
-template <int L, int P, int PAD, class Mul>
-__device__ __forceinline__ void fft_line_fwd_mul_inv(float2* buf, int stride, int lane, const float2* tw, bool active,
-                                                     Mul&& mul) {
-  constexpr int LAST = n_stages(L) - 1;
-  constexpr int RL = radix_of(L, LAST), NSL = L / RL, PER = (NSL + P - 1) / P;
-  ForwardStages<L, P, PAD, 0, LAST>::run(buf, stride, lane, tw, active);
-  float2 v[PER][RL];
-#pragma unroll
-  for (int b = 0; b < PER; ++b) {
-    const int j = lane + b * P;
-    if (active && (PER * P == NSL || j < NSL)) {
-#pragma unroll
-      for (int r = 0; r < RL; ++r) v[b][r] = buf[lpos<PAD>(j + r * NSL) * stride];
-      if constexpr (LAST > 0) {
-#pragma unroll
-        for (int r = 1; r < RL; ++r) v[b][r] = cmul(v[b][r], twiddle<-1>(tw, (r * j) % L));
-      }
-      Dft<RL, -1>::run(v[b]);
-#pragma unroll
-      for (int r = 0; r < RL; ++r) v[b][r] = mul(j + NSL * r, v[b][r]);
-      Dft<RL, 1>::run(v[b]);
-    }
-  }
-  __syncwarp();  // every lane has read the line before any writes it
-#pragma unroll
-  for (int b = 0; b < PER; ++b) {
-    const int j = lane + b * P;
-    if (active && (PER * P == NSL || j < NSL)) {
-#pragma unroll
-      for (int r = 0; r < RL; ++r) buf[lpos<PAD>(j * RL + r) * stride] = v[b][r];
-    }
-  }
-  __syncwarp();
-  InverseStagesReversed<L, P, PAD, LAST - 1, RL>::run(buf, stride, lane, tw, active);
-}
 
 // ---------------------------------------------------------------- lines across lanes
 // Mixed-radix stages for kernels whose neighbouring threads hold neighbouring lines: a thread has one
