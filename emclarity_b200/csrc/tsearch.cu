@@ -30,6 +30,7 @@ namespace emc {
 
 struct TsGeom {
   int nx, ny, nz, nxh;
+  int nxp;          // row pitch of the internal spectra: nxh rounded up to whole 32-byte sectors
   int t;            // template edge
   int pl[3];        // template offset inside the volume (BH_multi_padVal low pad)
   float m[9];       // sampling matrix rows
@@ -38,7 +39,7 @@ struct TsGeom {
 // Rotated template sampled into the x transforms of its rows: pair p of the t * ceil(t/2) row
 // pairs is rows (2q, 2q+1) of template plane zl; the line z[n] = a[n] + i b[n] holds the template
 // at x = n - pl[0] (zero outside), and the two half spectra go to rows pl[1] + 2q (+1) of plane zl
-// of ht ([t][ny][nxh]).  Sampling: 'forward' with shift [1,1,1], u = p - c - 1
+// of ht ([t][ny][nxp]).  Sampling: 'forward' with shift [1,1,1], u = p - c - 1
 // (BH_templateSearch3d_2.m:744), interpn-style trilinear.
 template <int L, int P>
 __global__ void __launch_bounds__(256) k_ts_rows(const float* __restrict__ tmpl, const TsGeom g,
@@ -87,8 +88,8 @@ __global__ void __launch_bounds__(256) k_ts_rows(const float* __restrict__ tmpl,
     __syncwarp();
     fft_line<L, -1, P, PAD>(buf, 1, lane, s_tw, active);
     if (active) {
-      float2* oa = ht + ((size_t)zl * g.ny + g.pl[1] + ya) * g.nxh;
-      float2* ob = oa + g.nxh;
+      float2* oa = ht + ((size_t)zl * g.ny + g.pl[1] + ya) * g.nxp;
+      float2* ob = oa + g.nxp;
       for (int k = lane; k <= L / 2; k += P) {
         const float2 zk = buf[lpos<PAD>(k)], zm = buf[lpos<PAD>((L - k) % L)];
         oa[k] = make_float2(0.5f * (zk.x + zm.x), 0.5f * (zk.y - zm.y));
@@ -177,13 +178,14 @@ __global__ void __launch_bounds__(ZfusedCfg<L>::T * ZfusedCfg<L>::P, ZfusedCfg<L
   float2* s_tw = smem;
   load_twiddles<L>(s_tw, g_tw);
   const int t = threadIdx.x % C::T, jt = threadIdx.x / C::T;
-  const long inner = (long)g.ny * g.nxh;
+  const long inner = (long)g.ny * g.nxp;
   const long i = (long)blockIdx.x * C::T + t;
-  const bool active = i < inner;
+  const int kx = (int)(i % g.nxp);
+  const bool active = i < inner && kx < g.nxh;  // (not the pad columns)
   const float2* gti = gt + i;
   const float2* ti = T + i;
   float2* si = s + i;
-  const double hw = ((int)(i % g.nxh) == 0 || 2 * (int)(i % g.nxh) == g.nx) ? 1.0 : 2.0;
+  const double hw = (kx == 0 || 2 * kx == g.nx) ? 1.0 : 2.0;
   float2* line = smem + L + t;
   __syncthreads();
   // Each thread sums its elements' |X|^2 in FP32 (L / P of them), the threads' sums are accumulated in
@@ -244,7 +246,7 @@ struct C2rMipSmem {
 };
 
 template <int L, int P>
-__global__ void __launch_bounds__(256) k_ts_c2r_mip(const float2* __restrict__ in, long nrows,
+__global__ void __launch_bounds__(256) k_ts_c2r_mip(const float2* __restrict__ in, long pitch, long nrows,
                                                     const double* __restrict__ stats, long nvox, float angle_id,
                                                     float* __restrict__ peak, float* __restrict__ angle,
                                                     const float2* __restrict__ g_tw) {
@@ -271,8 +273,8 @@ __global__ void __launch_bounds__(256) k_ts_c2r_mip(const float2* __restrict__ i
     if (pair < npairs) {
       const long ra = 2 * pair, rb = 2 * pair + 1;
       for (int k = lane; k < LH; k += P) {
-        cp_async8(sb + k, in + ra * LH + k);
-        if (rb < nrows) cp_async8(sb + LH + k, in + rb * LH + k);
+        cp_async8(sb + k, in + ra * pitch + k);
+        if (rb < nrows) cp_async8(sb + LH + k, in + rb * pitch + k);
       }
     }
     cp_async_commit();
@@ -338,16 +340,17 @@ __global__ void k_ts_init(float* __restrict__ peak, float* __restrict__ angle, l
 }
 
 __global__ void k_ts_ramp(float2* __restrict__ T, const float2* __restrict__ ex, const float2* __restrict__ ey,
-                          const float2* __restrict__ ez, int nxh, int ny, int nz) {
+                          const float2* __restrict__ ez, int nxh, int nxp, int ny, int nz) {
   const long total = (long)nz * ny * nxh;
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < total; i += (long)gridDim.x * blockDim.x) {
     const int x = (int)(i % nxh), y = (int)((i / nxh) % ny), z = (int)(i / ((long)nxh * ny));
-    T[i] = cmul(cmul(ex[x], ey[y]), cmul(ez[z], T[i]));
+    float2& v = T[((long)z * ny + y) * nxp + x];
+    v = cmul(cmul(ex[x], ey[y]), cmul(ez[z], v));
   }
 }
 
 template <int L>
-static emc_status launch_c2r_mip(const float2* in, long nrows, const double* stats, long nvox, float angle_id,
+static emc_status launch_c2r_mip(const float2* in, long pitch, long nrows, const double* stats, long nvox, float angle_id,
                                  float* peak, float* angle, cudaStream_t st) {
   constexpr int P = team_size(L);
   constexpr int TEAMS = rows_teams(L, P);
@@ -364,15 +367,15 @@ static emc_status launch_c2r_mip(const float2* in, long nrows, const double* sta
     attr_set[dev] = true;
   }
   const int grid = (int)std::max(1L, std::min((npairs + TEAMS - 1) / TEAMS, 8L * device_sm_count()));
-  k_ts_c2r_mip<L, P><<<grid, TEAMS * P, smem, st>>>(in, nrows, stats, nvox, angle_id, peak, angle, tw);
+  k_ts_c2r_mip<L, P><<<grid, TEAMS * P, smem, st>>>(in, pitch, nrows, stats, nvox, angle_id, peak, angle, tw);
   EMC_LAUNCH_CHECK();
   return EMC_OK;
 }
 
-static emc_status c2r_mip_any(int L, const float2* in, long nrows, const double* stats, long nvox, float angle_id,
+static emc_status c2r_mip_any(int L, const float2* in, long pitch, long nrows, const double* stats, long nvox, float angle_id,
                               float* peak, float* angle, cudaStream_t st) {
   switch (L) {
-#define X(n) case n: return launch_c2r_mip<n>(in, nrows, stats, nvox, angle_id, peak, angle, st);
+#define X(n) case n: return launch_c2r_mip<n>(in, pitch, nrows, stats, nvox, angle_id, peak, angle, st);
     EMC_FOR_EACH_LENGTH(X)
 #undef X
   }
@@ -418,7 +421,7 @@ static emc_status launch_ts_zfused(const float2* gt, const float2* T, float2* s,
     EMC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::smem));
     attr_set[dev] = true;
   }
-  const long inner = (long)g.ny * g.nxh;
+  const long inner = (long)g.ny * g.nxp;
   kern<<<(unsigned)((inner + C::T - 1) / C::T), C::T * C::P, C::smem, st>>>(gt, T, s, g, stats, tw);
   EMC_LAUNCH_CHECK();
   return EMC_OK;
@@ -439,10 +442,11 @@ static emc_status ts_zfused_any(int L, const float2* gt, const float2* T, float2
 
 struct emc_tsearch_s {
   int nx, ny, nz;
+  int nxp;                  // row pitch of every spectrum below
   float2* T = nullptr;      // tomogram spectrum with the phase ramp
   float2* G = nullptr;      // template spectrum / product
   float2* S = nullptr;      // C2R scratch
-  float2* ht = nullptr;     // x transforms of the template rows: [t][ny][nxh], other rows 0
+  float2* ht = nullptr;     // x transforms of the template rows: [t][ny][nxp], other rows 0
   int ht_t = 0;
   double* stats = nullptr;  // per orientation: sum |X|^2, X(0)
 };
@@ -459,14 +463,19 @@ emc_status emc_tsearch_create(const float* d_tomo, int nx, int ny, int nz, emc_t
   emc_tsearch_s* h = new (std::nothrow) emc_tsearch_s();
   EMC_CHECK_ARG(h, "emc_tsearch_create: host allocation failed");
   h->nx = nx; h->ny = ny; h->nz = nz;
-  const size_t nh = (size_t)(nx / 2 + 1) * ny * nz;
+  // rows of whole 32-byte sectors: the column passes' accesses are then aligned (257 columns are not)
+  h->nxp = (nx / 2 + 1 + 3) / 4 * 4;
+  const long nxp = h->nxp;
+  const size_t nh = (size_t)nxp * ny * nz;
   if (cudaMalloc(&h->T, nh * sizeof(float2)) || cudaMalloc(&h->G, nh * sizeof(float2)) ||
       cudaMalloc(&h->S, nh * sizeof(float2)) || cudaMalloc(&h->stats, 2 * sizeof(double))) {
     emc_tsearch_destroy(h);
     emc::set_error("emc_tsearch_create: device allocation failed");
     return EMC_E_OOM;
   }
-  emc_status rs = emc::fft3_r2c(d_tomo, h->T, nx, ny, nz, 1, st);
+  emc_status rs = emc::launch_rows_r2c(nx, d_tomo, nx, h->T, nxp, (long)ny * nz, st);
+  if (rs == EMC_OK) rs = emc::launch_cols(ny, -1, h->T, h->T, nxp, nxp, nz, ny * nxp, st);
+  if (rs == EMC_OK) rs = emc::launch_cols(nz, -1, h->T, h->T, ny * nxp, ny * nxp, 1, nz * ny * nxp, st);
   if (rs != EMC_OK) {
     emc_tsearch_destroy(h);
     return rs;
@@ -489,7 +498,7 @@ emc_status emc_tsearch_create(const float* d_tomo, int nx, int ny, int nz, emc_t
   EMC_CUDA(cudaMemcpyAsync(d_tab + ex.size() + ey.size(), ez.data(), ez.size() * sizeof(float2),
                            cudaMemcpyHostToDevice, st));
   emc::k_ts_ramp<<<4 * emc::device_sm_count(), 256, 0, st>>>(h->T, d_tab, d_tab + ex.size(),
-                                                             d_tab + ex.size() + ey.size(), nx / 2 + 1, ny, nz);
+                                                             d_tab + ex.size() + ey.size(), nx / 2 + 1, h->nxp, ny, nz);
   EMC_LAUNCH_CHECK();
   EMC_CUDA(cudaStreamSynchronize(st));  // host tables must outlive the copies
   cudaFreeAsync(d_tab, st);
@@ -503,19 +512,19 @@ emc_status emc_tsearch_run(emc_tsearch_t h, const float* d_template, int t, cons
   EMC_CHECK_ARG(t >= 1 && t <= h->nx && t <= h->ny && t <= h->nz, "emc_tsearch_run: template %d too large", t);
   EMC_CHECK_ARG(n_orient >= 1, "emc_tsearch_run: no orientations");
   cudaStream_t st = emc::as_stream(stream);
-  const int nx = h->nx, ny = h->ny, nz = h->nz, nxh = nx / 2 + 1;
+  const int nx = h->nx, ny = h->ny, nz = h->nz, nxh = nx / 2 + 1, nxp = h->nxp;
   const long nvox = (long)nx * ny * nz;
   if (h->ht_t != t) {
     if (h->ht) cudaFree(h->ht);
     h->ht = nullptr;
     h->ht_t = 0;
-    const size_t bytes = sizeof(float2) * (size_t)t * ny * nxh;
+    const size_t bytes = sizeof(float2) * (size_t)t * ny * nxp;
     EMC_CUDA(cudaMalloc(&h->ht, bytes));
     EMC_CUDA(cudaMemsetAsync(h->ht, 0, bytes, st));  // rows outside the template stay zero
     h->ht_t = t;
   }
   emc::TsGeom g;
-  g.nx = nx; g.ny = ny; g.nz = nz; g.nxh = nxh; g.t = t;
+  g.nx = nx; g.ny = ny; g.nz = nz; g.nxh = nxh; g.nxp = nxp; g.t = t;
   // BH_multi_padVal(t, n): low pad floor((n-t)/2) + (t odd) * ((n-t) odd)
   const int dims[3] = {nx, ny, nz};
   for (int a = 0; a < 3; ++a) g.pl[a] = (dims[a] - t) / 2 + ((t % 2) ? (dims[a] - t) % 2 : 0);
@@ -530,13 +539,13 @@ emc_status emc_tsearch_run(emc_tsearch_t h, const float* d_template, int t, cons
       for (int j = 0; j < 3; ++j) g.m[3 * i + j] = (float)M[i + 3 * j];
     // 1. rotated template sampled into the x transforms of its rows, 2. y transforms of its planes
     EMC_TRY(emc::ts_rows_any(nx, d_template, g, h->ht, st));
-    EMC_TRY(emc::launch_cols(ny, -1, h->ht, h->G, nxh, nxh, t, (long)ny * nxh, st));
+    EMC_TRY(emc::launch_cols(ny, -1, h->ht, h->G, nxp, nxp, t, (long)ny * nxp, st));
     // 3. z transform of the t planes, X = T conj(G) and its statistics, inverse z
     EMC_CUDA(cudaMemsetAsync(h->stats, 0, 2 * sizeof(double), st));
     EMC_TRY(emc::ts_zfused_any(nz, h->G, h->T, h->S, g, h->stats, st));
     // 4. inverse y, then C2R along x fused with std normalisation and the MIP update
-    EMC_TRY(emc::launch_cols(ny, 1, h->S, h->S, nxh, nxh, nz, (long)ny * nxh, st));
-    EMC_TRY(emc::c2r_mip_any(nx, h->S, (long)ny * nz, h->stats, nvox, (float)(o + 1), d_peak, d_angle, st));
+    EMC_TRY(emc::launch_cols(ny, 1, h->S, h->S, nxp, nxp, nz, (long)ny * nxp, st));
+    EMC_TRY(emc::c2r_mip_any(nx, h->S, nxp, (long)ny * nz, h->stats, nvox, (float)(o + 1), d_peak, d_angle, st));
   }
   return EMC_OK;
 }
