@@ -90,41 +90,6 @@ __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
 }
 
-// Pairs of FP32 values in one 64-bit register, and the packed multiply-add on them (sm_100): both
-// components round to nearest like fmaf.
-__device__ __forceinline__ unsigned long long pack2(float x, float y) {
-  unsigned long long d;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(x), "f"(y));
-  return d;
-}
-__device__ __forceinline__ float2 unpack2(unsigned long long v) {
-  float2 d;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(d.x), "=f"(d.y) : "l"(v));
-  return d;
-}
-__device__ __forceinline__ unsigned long long ffma2(unsigned long long a, unsigned long long b, unsigned long long c) {
-  unsigned long long d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-  return d;
-}
-
-__device__ __forceinline__ unsigned long long fmul2(unsigned long long a, unsigned long long b) {
-  unsigned long long d;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
-__device__ __forceinline__ unsigned long long fadd2(unsigned long long a, unsigned long long b) {
-  unsigned long long d;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
-// rounds towards minus infinity
-__device__ __forceinline__ unsigned long long fadd2_rd(unsigned long long a, unsigned long long b) {
-  unsigned long long d;
-  asm("add.rm.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
-
 // Bulk global -> shared copies through the tensor-memory-access unit (cp.async.bulk, this CTA's
 // own shared memory, no multicast), completed on a shared-memory mbarrier by transaction count.
 // Source and destination 16-byte aligned, size a multiple of 16.

@@ -35,6 +35,62 @@ __host__ __device__ __forceinline__ float2 mul_si(float2 a) {
   return SIGN < 0 ? make_float2(a.y, -a.x) : make_float2(-a.y, a.x);
 }
 
+#ifdef __CUDACC__
+// Pairs of FP32 values in one 64-bit register, and the packed multiply-add on them (sm_100): both
+// components round to nearest like fmaf.
+__device__ __forceinline__ unsigned long long pack2(float x, float y) {
+  unsigned long long d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(x), "f"(y));
+  return d;
+}
+__device__ __forceinline__ float2 unpack2(unsigned long long v) {
+  float2 d;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(d.x), "=f"(d.y) : "l"(v));
+  return d;
+}
+__device__ __forceinline__ unsigned long long ffma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+  unsigned long long d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+
+__device__ __forceinline__ unsigned long long fmul2(unsigned long long a, unsigned long long b) {
+  unsigned long long d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ unsigned long long fadd2(unsigned long long a, unsigned long long b) {
+  unsigned long long d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+// rounds towards minus infinity
+__device__ __forceinline__ unsigned long long fadd2_rd(unsigned long long a, unsigned long long b) {
+  unsigned long long d;
+  asm("add.rm.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+
+#endif
+// a + b, a - b and a + s b (s real) of complex values by packed instructions on the device: the same
+// roundings as the scalar forms in half the instructions (the arithmetic rate is the same, but the
+// transforms' kernels are short of issue slots).
+__host__ __device__ __forceinline__ float2 padd(float2 a, float2 b) {
+#ifdef __CUDA_ARCH__
+  return unpack2(fadd2(pack2(a.x, a.y), pack2(b.x, b.y)));
+#else
+  return cadd(a, b);
+#endif
+}
+__host__ __device__ __forceinline__ float2 pfma(float2 a, float s, float2 b) {
+#ifdef __CUDA_ARCH__
+  return unpack2(ffma2(pack2(b.x, b.y), pack2(s, s), pack2(a.x, a.y)));
+#else
+  return make_float2(fmaf(b.x, s, a.x), fmaf(b.y, s, a.y));
+#endif
+}
+__host__ __device__ __forceinline__ float2 psub(float2 a, float2 b) { return pfma(a, -1.f, b); }
+
 // cos / sin of rational multiples of pi used inside the codelets (exact math constants).
 #define EMC_SQRT1_2 0.70710678118654752440f
 #define EMC_COS_PI8 0.92387953251128675613f
@@ -71,11 +127,11 @@ template <int SIGN> struct Dft<3, SIGN> {
 
 template <int SIGN> struct Dft<4, SIGN> {
   static __host__ __device__ __forceinline__ void run(float2* v) {
-    float2 a0 = cadd(v[0], v[2]), a1 = csub(v[0], v[2]);
-    float2 b0 = cadd(v[1], v[3]), b1 = mul_si<SIGN>(csub(v[1], v[3]));
-    v[0] = cadd(a0, b0);
-    v[2] = csub(a0, b0);
-    v[1] = cadd(a1, b1);
+    float2 a0 = padd(v[0], v[2]), a1 = psub(v[0], v[2]);
+    float2 b0 = padd(v[1], v[3]), b1 = mul_si<SIGN>(psub(v[1], v[3]));
+    v[0] = padd(a0, b0);
+    v[2] = psub(a0, b0);
+    v[1] = cadd(a1, b1);  // (b1's components are swapped: no pair in registers)
     v[3] = csub(a1, b1);
   }
 };
@@ -86,14 +142,14 @@ template <int SIGN> struct Dft<8, SIGN> {
     float2 o[4] = {v[1], v[3], v[5], v[7]};
     Dft<4, SIGN>::run(e);
     Dft<4, SIGN>::run(o);
-    // w8^k = exp(SIGN 2 pi i k / 8)
-    float2 o1 = cscale(make_float2(o[1].x - (float)SIGN * o[1].y, o[1].y + (float)SIGN * o[1].x), EMC_SQRT1_2);
+    // w8^k = exp(SIGN 2 pi i k / 8); w8^1 o1 and w8^3 o3 without their factor 1 / sqrt 2
+    float2 o1 = make_float2(o[1].x - (float)SIGN * o[1].y, o[1].y + (float)SIGN * o[1].x);
     float2 o2 = mul_si<SIGN>(o[2]);
-    float2 o3 = cscale(make_float2(-o[3].x - (float)SIGN * o[3].y, -o[3].y + (float)SIGN * o[3].x), EMC_SQRT1_2);
-    v[0] = cadd(e[0], o[0]); v[4] = csub(e[0], o[0]);
-    v[1] = cadd(e[1], o1);   v[5] = csub(e[1], o1);
+    float2 o3 = make_float2(-o[3].x - (float)SIGN * o[3].y, -o[3].y + (float)SIGN * o[3].x);
+    v[0] = padd(e[0], o[0]); v[4] = psub(e[0], o[0]);
+    v[1] = pfma(e[1], EMC_SQRT1_2, o1); v[5] = pfma(e[1], -EMC_SQRT1_2, o1);
     v[2] = cadd(e[2], o2);   v[6] = csub(e[2], o2);
-    v[3] = cadd(e[3], o3);   v[7] = csub(e[3], o3);
+    v[3] = pfma(e[3], EMC_SQRT1_2, o3); v[7] = pfma(e[3], -EMC_SQRT1_2, o3);
   }
 };
 
@@ -118,8 +174,8 @@ template <int SIGN> struct Dft<16, SIGN> {
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
       float2 t = (k == 0) ? o[0] : cmul(o[k], w[k]);
-      v[k] = cadd(e[k], t);
-      v[k + 8] = csub(e[k], t);
+      v[k] = padd(e[k], t);
+      v[k + 8] = psub(e[k], t);
     }
   }
 };
