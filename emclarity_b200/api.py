@@ -45,6 +45,12 @@ def _dptr(arr):
     return arr, arr.ctypes.data_as(C.POINTER(C.c_double))
 
 
+def _doubles(values):
+    """values copied into a ctypes array of doubles (a few times cheaper to pass than a cast pointer)."""
+    a = np.array(values, dtype=np.float64, order="C")
+    return (C.c_double * a.size).from_buffer(a)
+
+
 # --------------------------------------------------------------------------- host math
 def define_matrix(angles, direction="inv"):
     """BH_defineMatrix(angles, 'Bah', direction) as a (3, 3) float64 array (row i, col j)."""
@@ -75,6 +81,9 @@ def search_matrices(phi_theta_psi, prior=None):
 
 
 # --------------------------------------------------------------------------- interpolator
+_floats3 = C.c_float * 3
+
+
 class Interpolator:
     """Rotate / shift / interpolate a volume (mexXform3d through interpolator.m).
 
@@ -98,14 +107,17 @@ class Interpolator:
         if m.size == 3:
             m = define_matrix(m, direction)
         m = m.reshape(3, 3)
-        mats = [m] if symmetry is None else [m @ s for s in symmetry]
-        packed = np.concatenate([np.asarray(x, dtype=np.float64).reshape(3, 3).flatten(order="F") for x in mats])
-        packed, pp = _dptr(packed)
-        sh = (C.c_float * 3)(*[float(v) for v in shifts])
+        # column-major operators, one after another
+        if symmetry is None:
+            count, pp = 1, _doubles(m.T)
+        else:
+            mats = np.asarray([m @ s for s in symmetry], dtype=np.float64).reshape(-1, 3, 3)
+            count, pp = len(mats), _doubles(mats.transpose(0, 2, 1))
+        sh = _floats3(*[float(v) for v in shifts])
         if out is None:
             out = torch.empty(self.shape, dtype=torch.float32, device="cuda")
         fwd = 1 if direction == "forward" else 0
-        L.call("emc_xform3d_apply", self._h, pp, len(mats), sh, fwd, self.interp, _need_cuda(out, "out"), _stream())
+        L.call("emc_xform3d_apply", self._h, pp, count, sh, fwd, self.interp, _need_cuda(out, "out"), _stream())
         return out
 
     def close(self):
@@ -556,8 +568,7 @@ class Average:
 
     def add(self, particles, rotations, halves, shifts=None, weights=None, wedges=None, wedge_index=None):
         k = particles.shape[0]
-        rot = np.ascontiguousarray(np.concatenate([np.asarray(r, np.float64).reshape(3, 3).flatten(order="F")
-                                                   for r in np.asarray(rotations).reshape(-1, 3, 3)]))
+        rot = _doubles(np.asarray(rotations, dtype=np.float64).reshape(-1, 3, 3).transpose(0, 2, 1))  # column-major
         hv = np.ascontiguousarray(halves, dtype=np.int32).reshape(k)
         sh = None if shifts is None else np.ascontiguousarray(shifts, dtype=np.float32).reshape(k, 3)
         wt = None if weights is None else np.ascontiguousarray(weights, dtype=np.float32).reshape(k)
@@ -569,7 +580,7 @@ class Average:
         fp = lambda a: None if a is None else a.ctypes.data_as(C.POINTER(C.c_float))
         ip = lambda a: None if a is None else a.ctypes.data_as(C.POINTER(C.c_int))
         L.call("emc_average_add", self._h, _need_cuda(particles, "particles"), k,
-               rot.ctypes.data_as(C.POINTER(C.c_double)), fp(sh), fp(wt), ip(hv), wp, nwdg, ip(wi), ip(kept),
+               rot, fp(sh), fp(wt), ip(hv), wp, nwdg, ip(wi), ip(kept),
                _stream())
         return kept.astype(bool)
 
