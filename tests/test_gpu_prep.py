@@ -81,3 +81,26 @@ def test_xcf_translational_matches_oracle(built_lib, cuda):
     assert np.array_equal(peak0, [3, -2, 1])
     scale = np.sqrt(np.sum(np.abs(R) ** 2 * np.where(np.arange(n // 2 + 1) % (n // 2) == 0, 1, 2)) * e)
     assert np.allclose(mp.cpu().numpy() * n ** 3 / scale, map_o, atol=1e-5 * np.abs(map_o).max())
+
+
+@pytest.mark.parametrize("n,count", [(2, 3), (6, 5), (16, 2), (48, 3), (90, 2), (126, 2), (144, 1)])
+def test_weighted_spectra_sizes(built_lib, cuda, n, count):
+    """Spectra weighted in the z transform, over line tiles with remainders and each kind of plan (one
+    stage, two, more; odd factors): against numpy in 64 bits with the transforms' tolerance, and the
+    energies against the sums of the returned spectra."""
+    from emclarity_b200 import api
+    rng = np.random.default_rng(n)
+    x = rng.standard_normal((count, n, n, n)).astype(np.float32)
+    w = rng.uniform(0.2, 1.5, (count, n, n, n // 2 + 1)).astype(np.float32)
+    b = rng.uniform(0.2, 1.5, (n, n, n // 2 + 1)).astype(np.float32)
+    q, e = api.particle_spectra(torch.from_numpy(x).cuda(), torch.from_numpy(w).cuda(), torch.from_numpy(b).cuda())
+    ref = np.fft.rfftn(x.astype(np.float64), axes=(1, 2, 3)) * w * b
+    ref[:, 0, 0, 0] = 0
+    got = q.cpu().numpy()
+    assert np.abs(got - ref).max() <= 2e-6 * np.abs(ref).max()
+    herm = np.full(n // 2 + 1, 2.0)
+    herm[0] = 1.0
+    if n % 2 == 0:
+        herm[-1] = 1.0
+    sums = ((got.real.astype(np.float64) ** 2 + got.imag.astype(np.float64) ** 2) * herm).sum(axis=(1, 2, 3))
+    assert np.allclose(e.cpu().numpy(), sums, rtol=1e-12)

@@ -507,3 +507,34 @@ def test_bounded_wait_reports_timeout_and_context_stays_usable(plain_case):
     s.status()
     assert np.array_equal(cc_d.cpu().numpy(), cc0)
     s.close()
+
+
+@pytest.mark.parametrize("store", ["f32", "bf16"])
+@pytest.mark.parametrize("n,radius,interp", [(64, 7, "linear"), (64, 8, "linear_border"), (96, 12, "linear"),
+                                             (96, 7, "linear_border"), (128, 7, "linear"), (128, 15, "linear_border")])
+def test_unmasked_noise_reference_reaches_every_edge(built_lib, cuda, n, radius, interp, store):
+    """A reference that is noise up to its faces and no mask: every brick edge and the inside test matter
+    (the identity samples exactly 0 and n - 1), shifts move the box, both ends of pass B's window
+    (narrow and wide radii) and a spectrum at an odd element offset.  Tolerance as everywhere."""
+    from emclarity_b200 import api
+    rng = np.random.default_rng(n + radius)
+    ref = rng.standard_normal((n, n, n)).astype(np.float32)
+    part = rng.standard_normal((n, n, n)).astype(np.float32)
+    grid = np.array([[0.0, 0.0, 0.0], [25.0, 50.0, -70.0], [200.0, 130.0, 11.0]])
+    shift = (1.5, -2.25, 0.75)
+    q, e = api.particle_spectrum(torch.from_numpy(part).cuda())
+    odd = torch.empty(q.numel() + 1, dtype=torch.complex64, device="cuda")[1:].view(q.shape)
+    odd.copy_(q)
+    s = api.Search(peak_radius=radius, interp=interp)
+    rid = s.add_reference(torch.from_numpy(ref).cuda(), store=store)
+    s.set_orientations(grid)
+    P, _ = O.particle_spectrum(part)
+    stored = torch.from_numpy(ref).bfloat16().float().numpy() if store == "bf16" else ref
+    kw = dict(interp={"linear": 0, "linear_border": 2}[interp])
+    mats = api.search_matrices(grid)
+    for sh in ((0.0, 0.0, 0.0), shift):
+        cc, pk, _ = s.run_host([s.particle(odd, e.item(), rid, shift=sh, orient_count=len(grid))])
+        cc_o, pk_o = O.search(stored, P, mats, radius=radius, shift=sh, **kw)
+        check_cc_and_peaks(cc, pk, cc_o, pk_o, lambda o: O.xcf_translational(stored, P, mats[o], shift=sh, **kw)[2],
+                           "n %d shift %s" % (n, sh))
+    s.close()
