@@ -30,6 +30,7 @@ struct AdjItem {
   const void* ref;      // n^3 reference (float or bf16)
   const void* cells;    // (n+1)^3 trilinear corner cells of the reference (same type) or null
   const float* mask;    // n^3 or null
+  const unsigned* mask_rows;  // x extents of the mask's non-zero voxels per (z, y) row, or null (see DevRef)
   const float* h;       // n^3 real-space particle template
   int n;
   int dtype;
@@ -37,36 +38,58 @@ struct AdjItem {
   AdjPose pose;
 };
 
+// Samplers work in two steps, so that several samples' loads are in flight before any is used.
 // Tricubic (Catmull-Rom) value and gradient from the plain volume.
 template <typename T>
 struct CubicSampler {
+  struct State {
+    float s[3];
+  };
   const T* ref;
   int n;
-  __device__ __forceinline__ float operator()(float sx, float sy, float sz, float g[3]) const {
-    return sample_cubic_grad(ref, n, n, n, sx, sy, sz, g);
+  __device__ __forceinline__ State start(float sx, float sy, float sz, bool) const { return {{sx, sy, sz}}; }
+  __device__ __forceinline__ float finish(const State& st, float g[3]) const {
+    return sample_cubic_grad(ref, n, n, n, st.s[0], st.s[1], st.s[2], g);
   }
 };
 
-// Trilinear value and gradient (interpn semantics, zero outside [0, n-1]) from the corner cells.
+// Trilinear value and gradient (interpn semantics, zero outside [0, n-1]) from the corner cells; a
+// sample outside (or one that nobody needs) loads no cell.
 template <typename T>
 struct CellSampler {
-  const CellT<T>* cells;
-  int n;
-  __device__ __forceinline__ float operator()(float sx, float sy, float sz, float g[3]) const {
+  struct State {
+    CellT<T> cell;
     float f[3];
     bool ok;
-    const long ci = cell_index<EMC_INTERP_LINEAR>(n, sx, sy, sz, f, &ok);
+  };
+  const CellT<T>* cells;
+  int n;
+  __device__ __forceinline__ State start(float sx, float sy, float sz, bool needed) const {
+    State st;
+    const float m = (float)(n - 1);
+    st.ok = needed && sx >= 0.f && sy >= 0.f && sz >= 0.f && sx <= m && sy <= m && sz <= m;
+    const float fx = __fadd_rd(sx, kFloorMagic), fy = __fadd_rd(sy, kFloorMagic), fz = __fadd_rd(sz, kFloorMagic);
+    st.f[0] = sx - (fx - kFloorMagic);
+    st.f[1] = sy - (fy - kFloorMagic);
+    st.f[2] = sz - (fz - kFloorMagic);
+    const unsigned nc = (unsigned)n + 1u, bias = 1u - kFloorBits;  // cell coordinates: floor + 1
+    const unsigned i = ((__float_as_uint(fz) + bias) * nc + __float_as_uint(fy) + bias) * nc + __float_as_uint(fx) + bias;
+    st.cell = load_cell_if(cells + i, st.ok);
+    return st;
+  }
+  __device__ __forceinline__ float finish(const State& st, float g[3]) const {
     float v[8];
-    cell_values(load_cell(cells + ci), v);
+    cell_values(st.cell, v);
+    const float* f = st.f;
     const float c00 = fmaf(f[0], v[1] - v[0], v[0]), c10 = fmaf(f[0], v[3] - v[2], v[2]);
     const float c01 = fmaf(f[0], v[5] - v[4], v[4]), c11 = fmaf(f[0], v[7] - v[6], v[6]);
     const float c0 = fmaf(f[1], c10 - c00, c00), c1 = fmaf(f[1], c11 - c01, c01);
     const float d0 = fmaf(f[1], (v[3] - v[2]) - (v[1] - v[0]), v[1] - v[0]);
     const float d1 = fmaf(f[1], (v[7] - v[6]) - (v[5] - v[4]), v[5] - v[4]);
-    g[0] = ok ? fmaf(f[2], d1 - d0, d0) : 0.f;
-    g[1] = ok ? fmaf(f[2], (c11 - c01) - (c10 - c00), c10 - c00) : 0.f;
-    g[2] = ok ? c1 - c0 : 0.f;
-    return ok ? fmaf(f[2], c1 - c0, c0) : 0.f;
+    g[0] = st.ok ? fmaf(f[2], d1 - d0, d0) : 0.f;
+    g[1] = st.ok ? fmaf(f[2], (c11 - c01) - (c10 - c00), c10 - c00) : 0.f;
+    g[2] = st.ok ? c1 - c0 : 0.f;
+    return st.ok ? fmaf(f[2], c1 - c0, c0) : 0.f;
   }
 };
 
@@ -77,10 +100,10 @@ __host__ __device__ inline bool adj_uses_cells(const AdjItem& it) {
   return it.interp == EMC_INTERP_LINEAR && it.cells != nullptr;
 }
 
-template <typename S>
+template <int U, typename S>
 __device__ __forceinline__ void adj_accumulate(const S sampler, const float* __restrict__ mask,
-                                               const float* __restrict__ h, int n, const AdjPose& sp,
-                                               float acc[kAdjSums]) {
+                                               const unsigned* __restrict__ mask_rows, const float* __restrict__ h,
+                                               int n, const AdjPose& sp, float acc[kAdjSums]) {
   const int c = n / 2;
   const int lane = threadIdx.x & 31;
   const int warps = (int)(gridDim.x * (blockDim.x >> 5));
@@ -90,40 +113,55 @@ __device__ __forceinline__ void adj_accumulate(const S sampler, const float* __r
     const float u1 = (float)(y - c) - sp.t[1], u2 = (float)(z - c) - sp.t[2];
     const float py = fmaf(m[1], u1, m[2] * u2), qy = fmaf(m[4], u1, m[5] * u2), ry = fmaf(m[7], u1, m[8] * u2);
     const long rbase = (long)row * n;
-    for (int x = lane; x < n; x += 32) {
-      const long i = rbase + x;
-      const float u0 = (float)(x - c) - sp.t[0];
-      const float sx = fmaf(m[0], u0, py) + (float)c;
-      const float sy = fmaf(m[3], u0, qy) + (float)c;
-      const float sz = fmaf(m[6], u0, ry) + (float)c;
-      const float mk = mask ? __ldg(mask + i) : 1.f;
-      if (mk == 0.f) continue;  // a zero mask voxel adds nothing to any of the sums
-      float g[3];
-      const float v = sampler(sx, sy, sz, g);
-      const float r = mk * v;
-      const float hv = __ldg(h + i);
-      g[0] *= mk; g[1] *= mk; g[2] *= mk;
-      acc[0] += r * hv;
-      acc[1] += r;
-      acc[2] += r * r;
-      // angle derivatives: ds/dk = dm_k u
+    const unsigned ext = mask_rows ? __ldg(mask_rows + row) : (unsigned)n << 16;
+    const int lo = (int)(ext & 0xffffu), hi = (int)(ext >> 16);
+    for (int x0 = lane; x0 < n; x0 += 32 * U) {
+      // U voxels' mask, template and sample loads together; a voxel outside the mask's extent on its row
+      // adds nothing to any of the sums and loads nothing
+      float mk[U], hv[U];
+      typename S::State st[U];
 #pragma unroll
-      for (int k = 0; k < 3; ++k) {
-        const float* d = sp.dm[k];
-        const float gk = g[0] * fmaf(d[0], u0, fmaf(d[1], u1, d[2] * u2)) +
-                         g[1] * fmaf(d[3], u0, fmaf(d[4], u1, d[5] * u2)) +
-                         g[2] * fmaf(d[6], u0, fmaf(d[7], u1, d[8] * u2));
-        acc[3 + 3 * k] += hv * gk;
-        acc[4 + 3 * k] += r * gk;
-        acc[5 + 3 * k] += gk;
+      for (int k = 0; k < U; ++k) {
+        const int x = x0 + 32 * k;
+        const bool in = x >= lo && x < hi;
+        const float u0 = (float)(x - c) - sp.t[0];
+        const float sx = fmaf(m[0], u0, py) + (float)c;
+        const float sy = fmaf(m[3], u0, qy) + (float)c;
+        const float sz = fmaf(m[6], u0, ry) + (float)c;
+        mk[k] = !in ? 0.f : mask ? __ldg(mask + rbase + x) : 1.f;
+        hv[k] = in ? __ldg(h + rbase + x) : 0.f;
+        st[k] = sampler.start(sx, sy, sz, in);
       }
-      // shift derivatives: ds/dt_j = -M[:, j]
 #pragma unroll
-      for (int j = 0; j < 3; ++j) {
-        const float gk = -(g[0] * m[j] + g[1] * m[3 + j] + g[2] * m[6 + j]);
-        acc[12 + 3 * j] += hv * gk;
-        acc[13 + 3 * j] += r * gk;
-        acc[14 + 3 * j] += gk;
+      for (int k = 0; k < U; ++k) {
+        if (mk[k] == 0.f) continue;  // a zero mask voxel adds nothing to any of the sums
+        const float u0 = (float)(x0 + 32 * k - c) - sp.t[0];
+        float g[3];
+        const float v = sampler.finish(st[k], g);
+        const float r = mk[k] * v;
+        g[0] *= mk[k]; g[1] *= mk[k]; g[2] *= mk[k];
+        acc[0] += r * hv[k];
+        acc[1] += r;
+        acc[2] += r * r;
+        // angle derivatives: ds/dk = dm_k u
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+          const float* d = sp.dm[q];
+          const float gk = g[0] * fmaf(d[0], u0, fmaf(d[1], u1, d[2] * u2)) +
+                           g[1] * fmaf(d[3], u0, fmaf(d[4], u1, d[5] * u2)) +
+                           g[2] * fmaf(d[6], u0, fmaf(d[7], u1, d[8] * u2));
+          acc[3 + 3 * q] += hv[k] * gk;
+          acc[4 + 3 * q] += r * gk;
+          acc[5 + 3 * q] += gk;
+        }
+        // shift derivatives: ds/dt_j = -M[:, j]
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+          const float gk = -(g[0] * m[j] + g[1] * m[3 + j] + g[2] * m[6 + j]);
+          acc[12 + 3 * j] += hv[k] * gk;
+          acc[13 + 3 * j] += r * gk;
+          acc[14 + 3 * j] += gk;
+        }
       }
     }
   }
@@ -134,7 +172,7 @@ __device__ __forceinline__ void adj_accumulate(const S sampler, const float* __r
 // each combination runs with the registers its own sampler needs (the tricubic sampler's gradient
 // needs far more than the trilinear one's).
 template <typename T, bool LIN>
-__global__ void __launch_bounds__(256) k_cc_adjoint(const AdjItem* __restrict__ items, double* __restrict__ sums) {
+__global__ void __launch_bounds__(256, LIN ? 2 : 1) k_cc_adjoint(const AdjItem* __restrict__ items, double* __restrict__ sums) {
   __shared__ AdjItem it;
   __shared__ double red[kAdjSums][8];
   const int item = blockIdx.y;
@@ -145,11 +183,19 @@ __global__ void __launch_bounds__(256) k_cc_adjoint(const AdjItem* __restrict__ 
   float acc[kAdjSums];
 #pragma unroll
   for (int k = 0; k < kAdjSums; ++k) acc[k] = 0.f;
-  if constexpr (LIN)
-    adj_accumulate(CellSampler<T>{reinterpret_cast<const CellT<T>*>(it.cells), it.n}, it.mask, it.h, it.n, it.pose,
-                   acc);
-  else
-    adj_accumulate(CubicSampler<T>{reinterpret_cast<const T*>(it.ref), it.n}, it.mask, it.h, it.n, it.pose, acc);
+  if constexpr (LIN) {
+    const CellSampler<T> sampler{reinterpret_cast<const CellT<T>*>(it.cells), it.n};
+    // a row's samples at once, or half a row's at 128^3: 3 in flight at 96^3 take 808 -> 693 us for 100
+    // items, although their registers leave two CTAs per SM instead of three (two at a time, a row and
+    // a half: 876 us; four at 128^3 spill)
+    if (it.n == 96)
+      adj_accumulate<3>(sampler, it.mask, it.mask_rows, it.h, 96, it.pose, acc);
+    else
+      adj_accumulate<2>(sampler, it.mask, it.mask_rows, it.h, it.n, it.pose, acc);
+  } else {
+    adj_accumulate<1>(CubicSampler<T>{reinterpret_cast<const T*>(it.ref), it.n}, it.mask, it.mask_rows, it.h, it.n,
+                      it.pose, acc);
+  }
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 #pragma unroll
   for (int k = 0; k < kAdjSums; ++k) {
@@ -222,7 +268,7 @@ static void pose_matrices(const double prior[9], const double* pose, AdjPose* ou
 
 // Defined in search.cu: access to a registered reference.
 emc_status emc_search_reference_info(emc_search_t s, int ref_id, const void** data, const void** cells,
-                                     const float** mask, int* n, int* dtype);
+                                     const float** mask, const unsigned** mask_rows, int* n, int* dtype);
 
 extern "C" {
 
@@ -241,12 +287,14 @@ emc_status emc_cc_adjoint_batch(emc_search_t s, int n_items, const int* ref_ids,
     const void* data = nullptr;
     const void* cells = nullptr;
     const float* mask = nullptr;
+    const unsigned* mask_rows = nullptr;
     int n = 0, dtype = 0;
-    EMC_TRY(emc_search_reference_info(s, ref_ids[i], &data, &cells, &mask, &n, &dtype));
+    EMC_TRY(emc_search_reference_info(s, ref_ids[i], &data, &cells, &mask, &mask_rows, &n, &dtype));
     items[i].ref = data;
     items[i].cells = cells;
     items[i].interp = interp;
     items[i].mask = mask;
+    items[i].mask_rows = mask_rows;
     items[i].h = d_h[i];
     items[i].n = n;
     items[i].dtype = dtype;
@@ -269,7 +317,7 @@ emc_status emc_cc_adjoint_batch(emc_search_t s, int n_items, const int* ref_ids,
   }
   if (rs == EMC_OK) {
     const long nv = (long)max_n * max_n * max_n;
-    // enough blocks per item to fill the GPU twice over (three trilinear CTAs fit per SM) without
+    // enough blocks per item to fill the GPU twice over (two trilinear CTAs fit per SM) without
     // starving the reduction
     const long want = std::max<long>(1, (8L * emc::device_sm_count() + n_items - 1) / n_items);
     const int bx = (int)std::max<long>(1, std::min<long>((nv + 2047) / 2048, want));

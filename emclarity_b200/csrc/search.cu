@@ -1023,13 +1023,14 @@ emc_status emc_particle_template(int n, const float* d_spectrum, float* d_h, voi
 
 // Read access to a registered reference (used by the adjoint entry point).
 emc_status emc_search_reference_info(emc_search_t s, int ref_id, const void** data, const void** cells,
-                                     const float** mask, int* n, int* dtype) {
+                                     const float** mask, const unsigned** mask_rows, int* n, int* dtype) {
   EMC_CHECK_ARG(s && data && cells && mask && n && dtype, "emc_search_reference_info: null argument");
   EMC_CHECK_ARG(ref_id >= 0 && ref_id < (int)s->refs.size(), "reference id %d not registered", ref_id);
   const auto& r = s->refs[ref_id];
   *data = r.data;
   *cells = r.cells;
   *mask = r.mask;
+  *mask_rows = r.mask_rows;
   *n = r.n;
   *dtype = r.dtype;
   return EMC_OK;

@@ -73,38 +73,24 @@ __device__ __forceinline__ void cell_values(const CellT<__nv_bfloat16>& c, float
     v[2 * i + 1] = f.y;
   }
 }
-// One 256-bit read-only load (sm_100): the whole 32-byte cell in a single request, so the cell's
-// sector is looked up once instead of once per 16-byte half.  Cells are 32-byte aligned.
-__device__ __forceinline__ CellT<float> load_cell(const CellT<float>* p) {
+// One 256-bit read-only load (sm_100) under a predicate: the whole 32-byte cell in a single request, so
+// the cell's sector is looked up once instead of once per 16-byte half.  Cells are 32-byte aligned.  An
+// inactive lane's value is undefined and its access is not made.
+__device__ __forceinline__ CellT<float> load_cell_if(const CellT<float>* p, bool on) {
   CellT<float> c;
-  asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+  asm volatile("{\n .reg .pred q;\n setp.ne.s32 q, %9, 0;\n"
+      " @q ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n}\n"
       : "=f"(c.lo.x), "=f"(c.lo.y), "=f"(c.lo.z), "=f"(c.lo.w), "=f"(c.hi.x), "=f"(c.hi.y), "=f"(c.hi.z),
         "=f"(c.hi.w)
-      : "l"(p));
+      : "l"(p), "r"((int)on));
   return c;
 }
-__device__ __forceinline__ CellT<__nv_bfloat16> load_cell(const CellT<__nv_bfloat16>* p) {
+__device__ __forceinline__ CellT<__nv_bfloat16> load_cell_if(const CellT<__nv_bfloat16>* p, bool on) {
   CellT<__nv_bfloat16> c;
-  c.v = __ldg(&p->v);
+  asm volatile("{\n .reg .pred q;\n setp.ne.s32 q, %5, 0;\n @q ld.global.nc.v4.u32 {%0, %1, %2, %3}, [%4];\n}\n"
+      : "=r"(c.v.x), "=r"(c.v.y), "=r"(c.v.z), "=r"(c.v.w)
+      : "l"(p), "r"((int)on));
   return c;
-}
-
-// Cell index and fractions of sample point s; `valid` follows interpn (MODE 0: 0 <= s <= n-1)
-// or the zero-border texture addressing (MODE 2: -1 < s < n).
-template <int MODE>
-__device__ __forceinline__ long cell_index(int n, float sx, float sy, float sz, float f[3], bool* valid) {
-  const bool ok = MODE == EMC_INTERP_LINEAR_BORDER
-                      ? (sx > -1.f && sy > -1.f && sz > -1.f && sx < (float)n && sy < (float)n && sz < (float)n)
-                      : (sx >= 0.f && sy >= 0.f && sz >= 0.f && sx <= (float)(n - 1) && sy <= (float)(n - 1) &&
-                         sz <= (float)(n - 1));
-  const float fx0 = floorf(sx), fy0 = floorf(sy), fz0 = floorf(sz);
-  const int x0 = max(-1, min((int)fx0, n - 1)), y0 = max(-1, min((int)fy0, n - 1)), z0 = max(-1, min((int)fz0, n - 1));
-  f[0] = sx - (float)x0;
-  f[1] = sy - (float)y0;
-  f[2] = sz - (float)z0;
-  *valid = ok;
-  const long nc = n + 1;
-  return ((long)(z0 + 1) * nc + (y0 + 1)) * nc + (x0 + 1);
 }
 
 // Pass A's copies.  A warp of pass A samples patches of 8 (y) x 4 (x) voxels of one plane, and what a
@@ -338,24 +324,6 @@ __device__ __forceinline__ float max_abs_nan(float a, float b, float c) {
       : "=f"(d)
       : "f"(a), "f"(b), "f"(c));
   return d;
-}
-
-// Cell load under a predicate; an inactive lane's value is undefined and its access is not made.
-__device__ __forceinline__ CellT<float> load_cell_if(const CellT<float>* p, bool on) {
-  CellT<float> c;
-  asm volatile("{\n .reg .pred q;\n setp.ne.s32 q, %9, 0;\n"
-      " @q ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n}\n"
-      : "=f"(c.lo.x), "=f"(c.lo.y), "=f"(c.lo.z), "=f"(c.lo.w), "=f"(c.hi.x), "=f"(c.hi.y), "=f"(c.hi.z),
-        "=f"(c.hi.w)
-      : "l"(p), "r"((int)on));
-  return c;
-}
-__device__ __forceinline__ CellT<__nv_bfloat16> load_cell_if(const CellT<__nv_bfloat16>* p, bool on) {
-  CellT<__nv_bfloat16> c;
-  asm volatile("{\n .reg .pred q;\n setp.ne.s32 q, %5, 0;\n @q ld.global.nc.v4.u32 {%0, %1, %2, %3}, [%4];\n}\n"
-      : "=r"(c.v.x), "=r"(c.v.y), "=r"(c.v.z), "=r"(c.v.w)
-      : "l"(p), "r"((int)on));
-  return c;
 }
 
 // Same interpolation order as sample_linear, so both paths give identical results.
