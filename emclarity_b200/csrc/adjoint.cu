@@ -185,7 +185,7 @@ __global__ void __launch_bounds__(256, LIN ? 2 : 1) k_cc_adjoint(const AdjItem* 
   for (int k = 0; k < kAdjSums; ++k) acc[k] = 0.f;
   if constexpr (LIN) {
     const CellSampler<T> sampler{reinterpret_cast<const CellT<T>*>(it.cells), it.n};
-    // a row's samples at once, or half a row's at 128^3: 3 in flight at 96^3 take 808 -> 693 us for 100
+    // a row's samples at once, or half a row's at 128^3: 3 in flight at 96^3 take 808 -> 577 us for 100
     // items, although their registers leave two CTAs per SM instead of three (two at a time, a row and
     // a half: 876 us; four at 128^3 spill)
     if (it.n == 96)

@@ -134,8 +134,9 @@ __global__ void __launch_bounds__(256) k_sf3d_images(const float4* __restrict__ 
 // memory, and then adds the listed columns for kSfVols volumes at once -- coalesced loads, no
 // divergence, no test repeated per voxel, and each output voxel written once (the summation over z
 // per column read and wrote it once per tilt).  128 volumes of 64^3 x 41 tilts: 372 us, their images
-// 48 us; the whole call 4,077 -> 553 us.  What is left waits for the columns' loads (L2 latency, eight
-// in flight per lane).  The block's minimum goes to min_key (an ordered key per volume) when given.
+// 48 us; the whole call 4,077 -> 553 us.  Four CTAs per SM instead of three (381 to 388 us)
+// or twice the loads in flight (377) change nothing: issue slots are 46 % busy, and warps with few tilts
+// wait for their CTA's busiest.  The block's minimum goes to min_key (an ordered key per volume) when given.
 constexpr int kSfX = 8;       // x positions (warps) per CTA: a row of 8 floats is one 32-byte sector
 constexpr int kSfList = 128;  // tilts listed at a time
 constexpr int kSfVols = 4;    // volumes per CTA

@@ -3,8 +3,7 @@
 //
 // A run evaluates every (particle, orientation) pair of the request.  Pairs are grouped by
 // (box size, reference storage type) and cut into chunks whose on-chip-spilled scratch
-// (S1 + S2) stays inside a budget sized to the L2 cache; each chunk is four launches
-// (fwd_xy, z_mul, inv_peak, decode).  The whole launch sequence of a run is captured once
+// (S1 + S2) stays inside a budget; each chunk is three launches (fwd_xy, z_mul, inv_peak).  The whole launch sequence of a run is captured once
 // in a CUDA graph; the graphs of the four most recent requests (particles, outputs, settings)
 // are kept, each with its own particle table, and replayed when a request repeats.
 #include <algorithm>
@@ -237,12 +236,12 @@ struct emc_search_s {
   emc::DevBuf<double> d_dmat;
   int norient = 0;
   int radius = 0, interp = EMC_INTERP_LINEAR, chunk_evals = 0;
-  // S1 + S2 scratch of a chunk: 768 MiB (about 600 evaluations at 64^3, 190 at 96^3, 84 at 128^3 with
-  // radius 7), or an eighth of the free device memory if that is less.  Measured: evaluations/s rise
-  // with the chunk until about this size (64^3: 370 k at 66 evaluations, the two-thirds-of-L2
-  // sizing, 400 k at 592, 403 k at 888; 96^3: 80 k at 21, 88 k at 168; 128^3: 31 k at 9, 34 k at
-  // 72): larger chunks amortise the passes' launch tails, and the slabs that then spill from L2
-  // cost HBM bandwidth the passes leave unused
+  // S1 + S2 scratch of a chunk: 768 MiB (about 545 evaluations at 64^3, 180 at 96^3, 80 at 128^3 with
+  // radius 7), or an eighth of the free device memory if that is less.  Larger chunks amortise the
+  // passes' launch tails, and the spectra that then spill from L2 cost HBM bandwidth the passes leave
+  // unused: one slot at 64^3 takes 2,402 ns per evaluation at 32 evaluations per chunk, 1,783 at 256,
+  // 1,731 at 520 (two slots: 1,828, 1,720, 1,712); 96^3 6,608 at 32, 5,641 at 192, 5,499 at 520; 128^3
+  // 14,173 at 32, 13,735 at 96, 13,416 at 520
   size_t scratch_budget = 768ull << 20;
 
   // Particle table and evaluation list of one recorded request.  Each cached graph reads its own
@@ -514,7 +513,7 @@ static int& planes_slot(emc_search_t s, int n, int dtype) {
 }
 
 // Times pass A on chunk c with every planes option that fits (one warm-up launch, then three
-// timed ones each) and stores the fastest. Pass A's outputs (S1 slabs, energy sums) are scratch
+// timed ones each) and stores the fastest. Pass A's outputs (S1, energy sums) are scratch
 // that the real run rewrites, so the trial launches leave no trace in the results.
 static emc_status tune_planes(emc_search_t s, const Chunk& c, cudaStream_t st) {
   const emc::SearchChunkArgs a = chunk_args(s, c);
@@ -574,9 +573,9 @@ static emc_status search_record(emc_search_t s, const std::vector<Chunk>& chunks
     ++launches;
   }
   // The second branch forks from the stream after the set-up above and joins before the outputs.
-  // Only 64^3 chunks overlap; larger ones run alone on the stream (the branch joined first): their
-  // passes fill the SMs by themselves, and beside another chunk's they ran slower (96^3: 96.0k
-  // evaluations/s with two slots against 101.1k with one; 128^3: 40.2k against 44.9k).
+  // Only 64^3 chunks overlap (1,712 against 1,729 ns per evaluation); larger ones run alone on the
+  // stream (the branch joined first): their passes fill the SMs by themselves, and beside another
+  // chunk's they lost 5 to 10 % when that was measured, with the passes of the time.
   const bool two = nslots > 1 && chunks.size() > 1;
   bool forked = false;
   long alternate = 0;

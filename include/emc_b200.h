@@ -326,7 +326,7 @@ EMC_API emc_status emc_search_run_host(emc_search_t s, const emc_particle_desc* 
                                emc_search_hit* h_best, void* stream);
 /* No counterpart in the reference.  Synchronises `stream` and reports whether a device-side wait of
  * the handle's runs since the last check gave up (EMC_E_TIMEOUT; the results of those runs are
- * invalid), clearing the report.  The waits (for the bulk copies of the z and peak passes) are bounded
+ * invalid), clearing the report.  The waits (for the bulk copies of the peak pass) are bounded
  * at about a second, after which the CTA leaves without a result; the context stays usable. */
 EMC_API emc_status emc_search_status(emc_search_t s, void* stream);
 /* Test hook (no counterpart in the reference): waits of later runs give up after wait_cycles SM
@@ -349,9 +349,9 @@ EMC_API emc_status emc_search_timings(emc_search_t s, double ms[4], long launche
 
 /* Tuning hook (no counterpart in the reference).  Pass A (rotate + xy R2C) runs planes = 1, 2, 4
  * or 8 z-planes per CTA.  Unless fixed here, the first emc_search_run that meets a (box, dtype)
- * times pass A on its first chunk with every planes value whose slab fits shared memory and
+ * times pass A on its first chunk with every planes value the box allows (up to 8, 4, 2) and
  * keeps the fastest for that handle.  emc_search_set_planes fixes the value for one box (both
- * dtypes; EMC_E_ARG if it does not divide the box or does not fit), 0 returns it to tuning.
+ * dtypes; EMC_E_ARG for a value the box does not allow), 0 returns it to tuning.
  * emc_search_get_planes reports the value in use for (box, dtype), 0 if not tuned yet, and the
  * pass-A time of each option at tuning (ms_per_option[k] for planes = 1 << k, -1 where not
  * timed; may be NULL). */
