@@ -507,10 +507,13 @@ emc_status mavg_ring(const float* in, float* vol, int nx, int ny, int nz, const 
   slab = std::max<long>(kMavgZ, slab / kMavgZ * kMavgZ);
   slab = std::min<long>(slab, nz);
   const int ring = (int)std::min<long>(nz, slab + L - 1);
-  const size_t smem = mavg_xy_smem<SQ>(L);
-  EMC_CUDA(cudaFuncSetAttribute(k_mavg_xy<SQ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  const size_t smem_z = mavg_z_smem<SQ>(L);
-  EMC_CUDA(cudaFuncSetAttribute(k_mavg_z<SQ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_z));
+  // the kernels' limits are those of the widest feature, not of this call's: threads with different
+  // features share them, and a smaller limit set between would refuse another thread's launch
+  const size_t smem = mavg_xy_smem<SQ>(L), smem_z = mavg_z_smem<SQ>(L);
+  EMC_CUDA(cudaFuncSetAttribute(k_mavg_xy<SQ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)mavg_xy_smem<SQ>(kMavgTaps)));
+  EMC_CUDA(cudaFuncSetAttribute(k_mavg_z<SQ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)mavg_z_smem<SQ>(kMavgTaps)));
   T* buf = nullptr;
   EMC_CUDA(cudaMallocAsync((void**)&buf, sizeof(T) * plane * ring, st));
   const dim3 tiles((nx + kMavgTile - 1) / kMavgTile, (ny + kMavgTile - 1) / kMavgTile);
