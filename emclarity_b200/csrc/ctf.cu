@@ -338,7 +338,7 @@ static emc_status sf3d_batch(const std::vector<SfTilt>& ts, const std::vector<fl
   const long npix = (long)nx * ny, nv = npix * nz;
   const size_t img_per = sizeof(float) * (size_t)n * npix;
   int chunk = (int)std::max<size_t>(1, std::min<size_t>((size_t)count, (size_t)(48ull << 20) / img_per));
-  chunk = std::min(count, (chunk + kSfVols - 1) / kSfVols * kSfVols);
+  chunk = std::min({count, (chunk + kSfVols - 1) / kSfVols * kSfVols, 65535 * kSfVols});  // (the grid's z extent)
   auto up = [](size_t b) { return (b + 255) / 256 * 256; };
   const size_t t_bytes = up(sizeof(SfTilt) * n), d_bytes = up(sizeof(float2) * df.size());
   const size_t k_bytes = up(sizeof(unsigned) * count), tab_bytes = up(sizeof(float4) * (size_t)n * npix);
