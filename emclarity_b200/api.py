@@ -48,6 +48,8 @@ def _dptr(arr):
 def _doubles(values):
     """values copied into a ctypes array of doubles (a few times cheaper to pass than a cast pointer)."""
     a = np.array(values, dtype=np.float64, order="C")
+    if a.size == 0:
+        raise ValueError("need at least one matrix")
     return (C.c_double * a.size).from_buffer(a)
 
 
