@@ -3,7 +3,8 @@
 //
 // A run evaluates every (particle, orientation) pair of the request.  Pairs are grouped by
 // (box size, reference storage type) and cut into chunks whose on-chip-spilled scratch
-// (S1 + S2) stays inside a budget; each chunk is three launches (fwd_xy, z_mul, inv_peak).  The whole launch sequence of a run is captured once
+// (S1 + S2) stays inside a budget; each chunk is three launches (fwd_xy, z_mul, inv_peak).  The whole
+// launch sequence of a run is captured once
 // in a CUDA graph; the graphs of the four most recent requests (particles, outputs, settings)
 // are kept, each with its own particle table, and replayed when a request repeats.
 #include <algorithm>
