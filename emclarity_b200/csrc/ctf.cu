@@ -11,6 +11,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "fft.cuh"
 
 namespace emc {
 
@@ -108,21 +109,67 @@ __global__ void k_sf3d_tables(const SfTilt* __restrict__ tilts, int nx, int ny, 
   tab[((long)blockIdx.z * nx + x) * ny + y] = v;
 }
 
-// The tilt images of `count` volumes, [volume][tilt][x][y] (lanes along y, as k_sf3d_volumes reads
-// them).  A thread keeps its pixel's table entry and walks the volumes: the radius, the angle and the
-// exposure filter, most of an image's arithmetic, are formed once per pixel instead of per volume.
+// Volumes whose image values lie together: K = 4 (a 16-byte load serves four volumes), or 1 for a
+// single volume.
+template <int K>
+struct SfVols;
+template <>
+struct SfVols<4> {
+  using Px = float4;
+  using W = unsigned long long;
+  unsigned long long a = 0ull, b = 0ull;  // two volumes a register pair, +0
+  static __device__ __forceinline__ W weight(float w) { return pack2(w, w); }
+  // += w ((1 - f) p + f q), g = 1 - f
+  __device__ __forceinline__ void add(const Px& p, const Px& q, W g, W f, W w) {
+    a = ffma2(w, ffma2(f, pack2(q.x, q.y), fmul2(g, pack2(p.x, p.y))), a);
+    b = ffma2(w, ffma2(f, pack2(q.z, q.w), fmul2(g, pack2(p.z, p.w))), b);
+  }
+  __device__ __forceinline__ float get(int v) const {
+    const float2 t = unpack2(v < 2 ? a : b);
+    return v & 1 ? t.y : t.x;
+  }
+  static __device__ __forceinline__ Px pixel(const float (&v)[4]) { return make_float4(v[0], v[1], v[2], v[3]); }
+};
+template <>
+struct SfVols<1> {
+  using Px = float;
+  using W = float;
+  float a = 0.f;
+  static __device__ __forceinline__ W weight(float w) { return w; }
+  __device__ __forceinline__ void add(Px p, Px q, W g, W f, W w) {
+    a = __fmaf_rn(w, __fmaf_rn(f, q, __fmul_rn(g, p)), a);
+  }
+  __device__ __forceinline__ float get(int) const { return a; }
+  static __device__ __forceinline__ Px pixel(const float (&v)[1]) { return v[0]; }
+};
+
+// The tilt images of `count` volumes, [group of K volumes][tilt][x][y][volume] and one column of zeros
+// after each group (lanes along y, as k_sf3d_volumes reads them).  A thread keeps its pixel's table
+// entry and walks the groups: the radius, the angle and the exposure filter, most of an image's
+// arithmetic, are formed once per pixel instead of per volume.
+template <int K>
 __global__ void __launch_bounds__(256) k_sf3d_images(const float4* __restrict__ tab, const SfTilt* __restrict__ tilts,
-                                                     const float2* __restrict__ df, int ntilts, long npix, int count,
-                                                     int squared, float* __restrict__ imgs) {
+                                                     const float2* __restrict__ df, int ntilts, long npix, int ny,
+                                                     int count, int squared, typename SfVols<K>::Px* __restrict__ imgs) {
   const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
   const int t = blockIdx.y;
   if (i >= npix) return;
   const float4 v = tab[(long)t * npix + i];
   const float amp = tilts[t].c.amp_phase;
-  for (int p = blockIdx.z; p < count; p += gridDim.z) {
-    const float2 d = __ldg(df + (long)p * ntilts + t);
-    const float s = sinf(v.x - v.y * (d.x + d.y * v.z) - amp);
-    imgs[((long)p * ntilts + t) * npix + i] = (squared ? s * s : s) * v.w;
+  const long ngroup = npix * ntilts + ny;
+  for (int g = blockIdx.z; g * K < count; g += gridDim.z) {
+    float val[K], none[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      val[k] = none[k] = 0.f;
+      if (g * K + k < count) {
+        const float2 d = __ldg(df + (long)(g * K + k) * ntilts + t);
+        const float s = sinf(v.x - v.y * (d.x + d.y * v.z) - amp);
+        val[k] = (squared ? s * s : s) * v.w;
+      }
+    }
+    imgs[g * ngroup + t * npix + i] = SfVols<K>::pixel(val);
+    if (t == 0 && i < ny) imgs[g * ngroup + ntilts * npix + i] = SfVols<K>::pixel(none);
   }
 }
 
@@ -131,41 +178,43 @@ __global__ void __launch_bounds__(256) k_sf3d_images(const float4* __restrict__ 
 // The plane tilts about y and its image rows are the volume's rows, so which tilts reach a voxel, the
 // two image columns they sample and their weights depend on (x, z) alone.  A warp takes one (x, z)
 // with its lanes along y: it tests the tilts 32 at a time, lists the few that reach it in shared
-// memory, and then adds the listed columns for kSfVols volumes at once -- coalesced loads, no
-// divergence, no test repeated per voxel, and each output voxel written once (the summation over z
-// per column read and wrote it once per tilt).  128 volumes of 64^3 x 41 tilts: 372 us, their images
-// 48 us; the whole call 4,077 -> 553 us.  Four CTAs per SM instead of three (381 to 388 us)
-// or twice the loads in flight (377) change nothing: issue slots are 46 % busy, and warps with few tilts
-// wait for their CTA's busiest.  The block's minimum goes to min_key (an ordered key per volume) when given.
+// memory, and then adds the listed columns for K volumes at once, group after group -- one coalesced
+// load per row brings the K volumes' values, columns outside the image are its zero column, each
+// output voxel is written once (the summation over z per column read and wrote it once per tilt).
+// 128 volumes of 64^3 x 41 tilts: 208 us, their images 50 us (372 and 48 us with an 8-byte load per
+// volume and two rows and an atomic per warp and volume for the minimum: those 262,144 atomics on 64 neighbouring
+// words were the bound); the whole call 4,023 -> 379 us (553).  What is left is the latency of the list, the loads and the barriers of short CTAs:
+// one group per CTA takes 212 us, six 244.
+// The block's minimum goes to min_key (an ordered key per volume) when given.
 constexpr int kSfX = 8;       // x positions (warps) per CTA: a row of 8 floats is one 32-byte sector
 constexpr int kSfList = 128;  // tilts listed at a time
-constexpr int kSfVols = 4;    // volumes per CTA
 
-// V: rows (consecutive y) per lane, 2 where the row count is even (8-byte loads, a 64-row image column
-// in one warp load), else 1.
-template <int V>
-__global__ void __launch_bounds__(32 * kSfX) k_sf3d_volumes(const float* __restrict__ imgs,
+// V: rows per lane, 32 apart (2, or 1 when there are no more than 32 rows).
+template <int V, int K>
+__global__ void __launch_bounds__(32 * kSfX, 3) k_sf3d_volumes(const typename SfVols<K>::Px* __restrict__ imgs,
                                                             const SfTilt* __restrict__ tilts, int ntilts, int count,
                                                             int nx, int ny, int nz, int zbase, float* __restrict__ out,
                                                             unsigned* __restrict__ min_key) {
-  __shared__ int2 s_col[kSfX][kSfList];    // offsets of the two image columns, -1: outside
+  using S = SfVols<K>;
+  __shared__ int2 s_col[kSfX][kSfList];    // the two image columns
   __shared__ float2 s_wt[kSfX][kSfList];   // (x fraction, edge weight)
-  __shared__ float s_out[kSfVols][32 * V][kSfX + 1];
+  __shared__ float s_out[K][32 * V][kSfX + 1];
+  __shared__ float s_low[K][kSfX];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int x = blockIdx.x * kSfX + warp, z = zbase + blockIdx.y, p0 = blockIdx.z * kSfVols;
-  const int nvol = min(kSfVols, count - p0);
-  const long npix = (long)nx * ny, nimg = npix * ntilts;
+  const int x = blockIdx.x * kSfX + warp, z = zbase + blockIdx.y;
+  const long ngroup = (long)nx * ny * ntilts + ny;
   const float PI = 3.14159265358979323f;
   const float ssx = (nx % 2 == 0) ? 0.5f : 0.f, ssz = (nz % 2 == 0) ? 0.5f : 0.f;
   const float u = (float)x - (float)nx / 2.0f;
   const float w = (float)(z - nz / 2);
+  const int none = ntilts * nx;  // the zero column
   // the tilts t0 .. t0 + kSfList - 1 that reach (x, z), in order; returns how many
   auto list = [&](int t0) {
     int n = 0;
     for (int tb = t0; tb < min(t0 + kSfList, ntilts); tb += 32) {
       const int t = tb + lane;
       bool hit = false;
-      int2 col = make_int2(-1, -1);
+      int2 col = make_int2(none, none);
       float2 wt = make_float2(0.f, 0.f);
       if (t < ntilts && x < nx) {
         const float sA = tilts[t].sinA, cA = tilts[t].cosA;
@@ -192,76 +241,72 @@ __global__ void __launch_bounds__(32 * kSfX) k_sf3d_volumes(const float* __restr
     __syncwarp();
     return n;
   };
-  const bool once = ntilts <= kSfList;  // one list serves every y
+  const bool once = ntilts <= kSfList;  // one list serves every y and every group
   int n = once ? list(0) : 0;
-  float low[kSfVols];
+  for (int g = blockIdx.z; g * K < count; g += gridDim.z) {
+    const int p0 = g * K, nvol = min(K, count - p0);
+    float low[K];
 #pragma unroll
-  for (int v = 0; v < kSfVols; ++v) low[v] = INFINITY;
-  for (int y0 = 0; y0 < ny; y0 += 32 * V) {
-    const int y = y0 + V * lane;
-    float acc[kSfVols][V];
+    for (int v = 0; v < K; ++v) low[v] = INFINITY;
+    for (int y0 = 0; y0 < ny; y0 += 32 * V) {
+      S acc[V];
+      // (lanes past the last row repeat it; what they form is not stored)
+      const typename S::Px* img[V];
 #pragma unroll
-    for (int v = 0; v < kSfVols; ++v)
-#pragma unroll
-      for (int q = 0; q < V; ++q) acc[v][q] = 0.f;
-    for (int t0 = 0; t0 < ntilts; t0 += kSfList) {
-      if (!once) {
-        __syncwarp();  // every lane is done with the previous list
-        n = list(t0);
-      }
-      // (lanes past the last row repeat it, volumes past the last one repeat the first; neither is stored)
-      const float* img = imgs + (long)p0 * nimg + min(y, ny - V);
-#pragma unroll 2
-      for (int k = 0; k < n; ++k) {
-        const int2 col = s_col[warp][k];
-        const float2 wt = s_wt[warp][k];
-        const long oa = (long)col.x * ny, ob = (long)col.y * ny;
-        float a[kSfVols][V], b[kSfVols][V];
-#pragma unroll
-        for (int v = 0; v < kSfVols; ++v) {
-          const float* iv = img + (v < nvol ? v * nimg : 0);
-          if constexpr (V == 2) {
-            const float2 zero = make_float2(0.f, 0.f);
-            const float2 fa = col.x >= 0 ? __ldg(reinterpret_cast<const float2*>(iv + oa)) : zero;
-            const float2 fb = col.y >= 0 ? __ldg(reinterpret_cast<const float2*>(iv + ob)) : zero;
-            a[v][0] = fa.x; a[v][1] = fa.y;
-            b[v][0] = fb.x; b[v][1] = fb.y;
-          } else {
-            a[v][0] = col.x >= 0 ? __ldg(iv + oa) : 0.f;
-            b[v][0] = col.y >= 0 ? __ldg(iv + ob) : 0.f;
-          }
+      for (int q = 0; q < V; ++q) img[q] = imgs + g * ngroup + min(y0 + lane + 32 * q, ny - 1);
+      for (int t0 = 0; t0 < ntilts; t0 += kSfList) {
+        if (!once) {
+          __syncwarp();  // every lane is done with the previous list
+          n = list(t0);
         }
+#pragma unroll 2
+        for (int k = 0; k < n; ++k) {
+          const int2 col = s_col[warp][k];
+          const float2 wt = s_wt[warp][k];
+          const long oa = (long)col.x * ny, ob = (long)col.y * ny;
+          typename S::Px a[V], b[V];
 #pragma unroll
-        for (int v = 0; v < kSfVols; ++v)
+          for (int q = 0; q < V; ++q) {
+            a[q] = __ldg(img[q] + oa);
+            b[q] = __ldg(img[q] + ob);
+          }
+          const typename S::W wg = S::weight(1.f - wt.x), wf = S::weight(wt.x), we = S::weight(wt.y);
 #pragma unroll
-          for (int q = 0; q < V; ++q) acc[v][q] += wt.y * ((1.f - wt.x) * a[v][q] + wt.x * b[v][q]);
+          for (int q = 0; q < V; ++q) acc[q].add(a[q], b[q], wg, wf, we);
+        }
       }
-    }
-#pragma unroll
-    for (int v = 0; v < kSfVols; ++v)
-#pragma unroll
-      for (int q = 0; q < V; ++q) s_out[v][V * lane + q][warp] = acc[v][q];
-    __syncthreads();
-    for (int i = threadIdx.x; i < nvol * 32 * V * kSfX; i += blockDim.x) {
-      const int c = i % kSfX, r = (i / kSfX) % (32 * V), v = i / (kSfX * 32 * V);
-      const int xo = blockIdx.x * kSfX + c, yo = y0 + r;
-      if (xo < nx && yo < ny) out[(((long)(p0 + v) * nz + z) * ny + yo) * nx + xo] = s_out[v][r][c];
-    }
-    __syncthreads();
-#pragma unroll
-    for (int v = 0; v < kSfVols; ++v)
 #pragma unroll
       for (int q = 0; q < V; ++q)
-        if (x < nx && y + q < ny) low[v] = fminf(low[v], acc[v][q]);  // NaN never becomes the minimum
-  }
-  if (!min_key) return;
 #pragma unroll
-  for (int v = 0; v < kSfVols; ++v) {
-    if (v >= nvol) break;
-    float m = low[v];
+        for (int v = 0; v < K; ++v) {
+          const float val = acc[q].get(v);
+          s_out[v][lane + 32 * q][warp] = val;
+          if (x < nx && y0 + lane + 32 * q < ny) low[v] = fminf(low[v], val);  // NaN never becomes the minimum
+        }
+      __syncthreads();
+      for (int i = threadIdx.x; i < nvol * 32 * V * kSfX; i += blockDim.x) {
+        const int c = i % kSfX, r = (i / kSfX) % (32 * V), v = i / (kSfX * 32 * V);
+        const int xo = blockIdx.x * kSfX + c, yo = y0 + r;
+        if (xo < nx && yo < ny) out[(((long)(p0 + v) * nz + z) * ny + yo) * nx + xo] = s_out[v][r][c];
+      }
+      __syncthreads();
+    }
+    if (!min_key) continue;
+    // one atomic per CTA and volume: the keys share a few sectors, whose atomics run one after another
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) m = fminf(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if (lane == 0 && m < INFINITY) atomicMin(min_key + p0 + v, ordered_key(m));
+    for (int v = 0; v < K; ++v) {
+      float m = low[v];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) m = fminf(m, __shfl_xor_sync(0xffffffffu, m, o));
+      if (lane == 0) s_low[v][warp] = m;
+    }
+    __syncthreads();
+    if (threadIdx.x < nvol) {
+      float m = s_low[threadIdx.x][0];
+#pragma unroll
+      for (int q = 1; q < kSfX; ++q) m = fminf(m, s_low[threadIdx.x][q]);
+      if (m < INFINITY) atomicMin(min_key + p0 + threadIdx.x, ordered_key(m));
+    }
   }
 }
 
@@ -331,14 +376,16 @@ __global__ void k_vol_sub_min(float* __restrict__ v, long n, const unsigned* __r
 
 // SF3D volumes of a batch: tilts ts (shared), defocus pairs df [volume][tilt]; `shifted` subtracts
 // min - 1e-4 from each.  Volumes go through in chunks whose tilt images (and so, at the usual 40
-// tilts, volumes) stay in the L2 between the launches.
+// tilts, volumes) stay in the L2 between the launches.  K: volumes per group.
+template <int K>
 static emc_status sf3d_batch(const std::vector<SfTilt>& ts, const std::vector<float2>& df, int count, int nx, int ny,
                              int nz, int squared, bool shifted, float* d_out, cudaStream_t st) {
+  using Px = typename SfVols<K>::Px;
   const int n = (int)ts.size();
   const long npix = (long)nx * ny, nv = npix * nz;
-  const size_t img_per = sizeof(float) * (size_t)n * npix;
-  int chunk = (int)std::max<size_t>(1, std::min<size_t>((size_t)count, (size_t)(48ull << 20) / img_per));
-  chunk = std::min({count, (chunk + kSfVols - 1) / kSfVols * kSfVols, 65535 * kSfVols});  // (the grid's z extent)
+  const size_t group = sizeof(Px) * ((size_t)n * npix + ny);  // bytes of a group's images
+  const int ngroups = (count + K - 1) / K;
+  const int chunk = (int)std::max<size_t>(1, std::min<size_t>({(size_t)ngroups, (size_t)(48ull << 20) / group, 65535}));
   auto up = [](size_t b) { return (b + 255) / 256 * 256; };
   const size_t t_bytes = up(sizeof(SfTilt) * n), d_bytes = up(sizeof(float2) * df.size());
   const size_t k_bytes = up(sizeof(unsigned) * count), tab_bytes = up(sizeof(float4) * (size_t)n * npix);
@@ -346,33 +393,38 @@ static emc_status sf3d_batch(const std::vector<SfTilt>& ts, const std::vector<fl
   memcpy(host.data(), ts.data(), sizeof(SfTilt) * n);
   memcpy(host.data() + t_bytes, df.data(), sizeof(float2) * df.size());
   char* buf = nullptr;
-  EMC_CUDA(cudaMallocAsync(&buf, t_bytes + d_bytes + k_bytes + tab_bytes + img_per * chunk, st));
+  EMC_CUDA(cudaMallocAsync(&buf, t_bytes + d_bytes + k_bytes + tab_bytes + group * chunk, st));
   const SfTilt* d_t = reinterpret_cast<const SfTilt*>(buf);
   const float2* d_df = reinterpret_cast<const float2*>(buf + t_bytes);
   unsigned* keys = reinterpret_cast<unsigned*>(buf + t_bytes + d_bytes);
   float4* tab = reinterpret_cast<float4*>(buf + t_bytes + d_bytes + k_bytes);
-  float* imgs = reinterpret_cast<float*>(buf + t_bytes + d_bytes + k_bytes + tab_bytes);
+  Px* imgs = reinterpret_cast<Px*>(buf + t_bytes + d_bytes + k_bytes + tab_bytes);
   cudaError_t e = cudaMemcpyAsync(buf, host.data(), host.size(), cudaMemcpyHostToDevice, st);
   if (e == cudaSuccess && shifted) e = cudaMemsetAsync(keys, 0xff, sizeof(unsigned) * count, st);
   if (e == cudaSuccess) {
     k_sf3d_tables<<<dim3((ny + 31) / 32, (nx + 7) / 8, n), dim3(32, 8), 0, st>>>(d_t, nx, ny, tab);
     e = cudaGetLastError();
   }
-  for (int p0 = 0; p0 < count && e == cudaSuccess; p0 += chunk) {
-    const int cnt = std::min(chunk, count - p0);
+  for (int g0 = 0; g0 < ngroups && e == cudaSuccess; g0 += chunk) {
+    const int p0 = g0 * K, cnt = std::min(chunk * K, count - p0), gs = (cnt + K - 1) / K;
     float* out = d_out + (size_t)p0 * nv;
-    // enough volumes side by side to fill the chip when one volume's pixels do not
+    // enough groups side by side to fill the chip when one group's pixels do not
     const unsigned blocks = (unsigned)((npix + 255) / 256);
-    const unsigned zs = (unsigned)std::min<long>(cnt, 1 + 16L * device_sm_count() / ((long)blocks * n));
-    k_sf3d_images<<<dim3(blocks, n, zs), 256, 0, st>>>(tab, d_t, d_df + (size_t)p0 * n, n, npix, cnt, squared, imgs);
-    for (int z0 = 0; z0 < nz; z0 += 65535)
-      (ny % 2 == 0 ? k_sf3d_volumes<2> : k_sf3d_volumes<1>)<<<
-          dim3((nx + kSfX - 1) / kSfX, std::min(nz - z0, 65535), (cnt + kSfVols - 1) / kSfVols), 32 * kSfX, 0, st>>>(
+    const unsigned zs = (unsigned)std::min<long>(gs, 1 + 16L * device_sm_count() / ((long)blocks * n));
+    k_sf3d_images<K><<<dim3(blocks, n, zs), 256, 0, st>>>(tab, d_t, d_df + (size_t)p0 * n, n, npix, ny, cnt, squared, imgs);
+    const unsigned gx = (nx + kSfX - 1) / kSfX;
+    for (int z0 = 0; z0 < nz; z0 += 65535) {
+      // a CTA's list serves as many groups as leave about eight waves of CTAs (two groups at 64 volumes of 64^3)
+      const int gy = std::min(nz - z0, 65535);
+      const long per = std::max<long>(1, std::min<long>(gs, (long)gx * gy * gs / (24L * device_sm_count())));
+      (ny > 32 ? k_sf3d_volumes<2, K> : k_sf3d_volumes<1, K>)<<<dim3(gx, gy, (unsigned)((gs + per - 1) / per)),
+                                                                 32 * kSfX, 0, st>>>(
           imgs, d_t, n, cnt, nx, ny, nz, z0, out, shifted ? keys + p0 : nullptr);
+    }
     if (shifted) {
-      const int gx = (int)std::max<long>(1, std::min<long>((nv + 1023) / 1024, 64));
+      const int gxm = (int)std::max<long>(1, std::min<long>((nv + 1023) / 1024, 64));
       for (int q = 0; q < cnt; q += 65535)
-        k_vol_sub_min<<<dim3(gx, std::min(cnt - q, 65535)), 256, 0, st>>>(out + (size_t)q * nv, nv, keys + p0 + q, 1e-4f);
+        k_vol_sub_min<<<dim3(gxm, std::min(cnt - q, 65535)), 256, 0, st>>>(out + (size_t)q * nv, nv, keys + p0 + q, 1e-4f);
     }
     e = cudaGetLastError();
   }
@@ -457,7 +509,7 @@ emc_status emc_sf3d(int half, int squared, const unsigned size[3], const float* 
     ts[t].occ = occupancy[t];
     ts[t].expo = exposure[t];
   }
-  return emc::sf3d_batch(ts, df, 1, nx, ny, nz, squared, false, d_out, emc::as_stream(stream));
+  return emc::sf3d_batch<1>(ts, df, 1, nx, ny, nz, squared, false, d_out, emc::as_stream(stream));
 }
 
 // BH_weightMaskMex(SIZE, SAMPLING, TLT, xyzSubTomo, reconGeometry) for a batch of particles
@@ -533,7 +585,8 @@ emc_status emc_sf3d_particles(const unsigned size[3], double sampling, const dou
       df[(size_t)p * n + r] = make_float2(0.5f * (d1 + d2), 0.5f * (d1 - d2));
     }
   }
-  return emc::sf3d_batch(ts, df, count, nx, ny, nz, 1, true, d_out, emc::as_stream(stream));
+  return (count > 1 ? emc::sf3d_batch<4> : emc::sf3d_batch<1>)(ts, df, count, nx, ny, nz, 1, true, d_out,
+                                                                emc::as_stream(stream));
 }
 
 }  // extern "C"
