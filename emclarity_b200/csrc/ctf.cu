@@ -181,10 +181,11 @@ __global__ void __launch_bounds__(256) k_sf3d_images(const float4* __restrict__ 
 // memory, and then adds the listed columns for K volumes at once, group after group -- one coalesced
 // load per row brings the K volumes' values, columns outside the image are its zero column, each
 // output voxel is written once (the summation over z per column read and wrote it once per tilt).
-// 128 volumes of 64^3 x 41 tilts: 208 us, their images 50 us (372 and 48 us with an 8-byte load per
-// volume and two rows and an atomic per warp and volume for the minimum: those 262,144 atomics on 64 neighbouring
-// words were the bound); the whole call 4,023 -> 379 us (553).  What is left is the latency of the list, the loads and the barriers of short CTAs:
-// one group per CTA takes 212 us, six 244.
+// 128 volumes of 64^3 x 41 tilts: 208 us, their images 50 us, the whole call 4,023 -> 379 us.  With an
+// 8-byte load per volume and two rows, and an atomic per warp and volume for the minimum, the sums took
+// 372 us and the call 553: 262,144 atomics per launch on some 64 neighbouring words were the bound.  What
+// is left is the latency of the list, the loads and the barriers of short CTAs: one group per CTA takes
+// 212 us, six 244.
 // The block's minimum goes to min_key (an ordered key per volume) when given.
 constexpr int kSfX = 8;       // x positions (warps) per CTA: a row of 8 floats is one 32-byte sector
 constexpr int kSfList = 128;  // tilts listed at a time
