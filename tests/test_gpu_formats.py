@@ -139,3 +139,20 @@ def test_sf3d_particles_sizes(built_lib, cuda, size, tilts, count):
     ref = O.sf3d_particles_np(size, 2.0, t, xyz, rg)
     for g, r in zip(got, ref):
         assert np.abs(g - r).max() <= 2e-4 * np.abs(r).max(), np.abs(g - r).max()
+
+
+@pytest.mark.parametrize("ny,tilts", [(4, 3), (34, 130)])
+def test_sf3d_particles_several_groups_per_list(built_lib, cuda, ny, tilts):
+    """Enough positions and volumes that a CTA's tilt list serves several groups of volumes, with one list
+    for all tilts and with several; same tolerance as the cubic case."""
+    from emclarity_b200 import api
+    rng = np.random.default_rng(tilts)
+    t = _tilt_table(rng, tilts)
+    rg = np.array([[512, 512, 256], [0.0, 1.0, -2.0]])
+    size, count = (9, ny, 512), 57
+    xyz = rng.uniform(1, [512, 512, 256], (count, 3))
+    got = api.sf3d_particles(size, 2.0, t, xyz, rg).cpu().numpy()
+    pick = [0, 3, 4, 31, 55, 56]
+    ref = O.sf3d_particles_np(size, 2.0, t, xyz[pick], rg)
+    for p, r in zip(pick, ref):
+        assert np.abs(got[p] - r).max() <= 2e-4 * np.abs(r).max(), (p, np.abs(got[p] - r).max())
