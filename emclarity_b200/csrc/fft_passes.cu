@@ -52,7 +52,7 @@ static emc_status cols_t(const float2* in, float2* out, long stride, long inner,
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 64) return EMC_E_CUDA;
-  if (C::smem > 48 * 1024 && !ready[dev].load(std::memory_order_acquire)) {
+  if (C::opt_in && !ready[dev].load(std::memory_order_acquire)) {
     EMC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::smem));
     ready[dev].store(true, std::memory_order_release);
   }
@@ -128,7 +128,7 @@ static emc_status cols_weighted_t(float2* q, int count, const float* wgt, const 
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 64) return EMC_E_CUDA;
-  if (C::smem > 48 * 1024 && !ready[dev].load(std::memory_order_acquire)) {
+  if (C::opt_in && !ready[dev].load(std::memory_order_acquire)) {
     EMC_CUDA(cudaFuncSetAttribute(k_cols_weighted<L>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::smem));
     ready[dev].store(true, std::memory_order_release);
   }

@@ -104,6 +104,11 @@ __global__ void __launch_bounds__(256) k_rows_c2r(const float2* __restrict__ in,
   }
 }
 
+// Whether a launch with this much dynamic shared memory needs the opt-in attribute: the 48 KiB that a
+// kernel has without it also hold what the kernel declares statically (at most 1 KiB here; 360-point
+// lines take 48,960 dynamic bytes, and with 256 static ones their launch was refused).
+constexpr bool needs_smem_opt_in(size_t dynamic) { return dynamic + 1024 > 48 * 1024; }
+
 // ----------------------------------------------------------------- strided columns
 // Complex lines along a strided axis: element n of line (o, i) lives at
 // base + o*outer_pitch + i + n*stride, for i in [0, inner), o in [0, outer); in == out is allowed.
@@ -130,6 +135,7 @@ struct ColsCfg {
   static constexpr int J = best(MOST / 4 + MOST / 4 % 2 > 2 ? MOST / 4 + MOST / 4 % 2 : 2,
                                 MOST / 4 + MOST / 4 % 2 > 2 ? MOST / 4 + MOST / 4 % 2 : 2);
   static constexpr size_t smem = sizeof(float2) * (L + (size_t)L * T);
+  static constexpr bool opt_in = needs_smem_opt_in(smem);
   static constexpr int by_smem = (int)((220 * 1024) / (smem + 1024));
   static constexpr int by_regs = 1024 / (T * J) > 1 ? 1024 / (T * J) : 1;  // 64 registers a thread
   static constexpr int min_blocks = by_smem < by_regs ? by_smem : by_regs;

@@ -362,7 +362,7 @@ static emc_status launch_c2r_mip(const float2* in, long pitch, long nrows, const
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 64) return EMC_E_CUDA;
-  if (smem > 48 * 1024 && !attr_set[dev]) {
+  if (needs_smem_opt_in(smem) && !attr_set[dev]) {
     EMC_CUDA(cudaFuncSetAttribute(k_ts_c2r_mip<L, P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     attr_set[dev] = true;
   }
@@ -417,7 +417,7 @@ static emc_status launch_ts_zfused(const float2* gt, const float2* T, float2* s,
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 64) return EMC_E_CUDA;
-  if (C::smem > 48 * 1024 && !attr_set[dev]) {
+  if (needs_smem_opt_in(C::smem) && !attr_set[dev]) {
     EMC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::smem));
     attr_set[dev] = true;
   }

@@ -105,3 +105,20 @@ def test_template_search_finds_planted_particles(built_lib, cuda):
     for (z, y, x), _ in pos:
         win = peak[z - 2:z + 3, y - 2:y + 3, x - 2:x + 3]
         assert win.max() > np.percentile(peak, 99.9)
+
+
+@pytest.mark.parametrize("nz", [320, 336, 360, 378])
+def test_template_search_z_lengths_at_the_shared_memory_limit(built_lib, cuda, nz):
+    """z edges on both sides of the 48 KiB that a launch has without an opt-in (360 lies inside it by its
+    line tiles alone, and beyond with the kernel's static part)."""
+    from emclarity_b200 import api, synthetic
+    rng = np.random.default_rng(nz)
+    tmpl = synthetic.blob_reference(rng, 8, n_blobs=4)
+    tomo = rng.standard_normal((nz, 16, 24)).astype(np.float32)
+    grid = np.array([[0.0, 0.0, 0.0], [30.0, 60.0, -40.0]])
+    ts = api.TemplateSearch(torch.from_numpy(tomo).cuda())
+    peak, ang = ts.run(torch.from_numpy(tmpl).cuda(), grid)
+    ts.close()
+    mats = [api.define_matrix([p, th, ps - p], "forward") for p, th, ps in grid]
+    maps, peak_o, ang_o = oracle_maps(tomo, tmpl, mats)
+    check_mip(peak.cpu().numpy(), ang.cpu().numpy(), maps, peak_o, ang_o)
