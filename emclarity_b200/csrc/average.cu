@@ -198,9 +198,14 @@ __global__ void __launch_bounds__(256, 3) k_avg_rotate(const float* __restrict__
     bool fits = true;
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
+      const float ax = fabsf(m[3 * i]), ay = fabsf(m[3 * i + 1]), az = fabsf(m[3 * i + 2]);
       const float mid = m[3 * i] * cu + m[3 * i + 1] * cv + m[3 * i + 2] * cw + sh[i] + (float)c;
-      const float ext = fabsf(m[3 * i]) * hx + fabsf(m[3 * i + 1]) * hy + fabsf(m[3 * i + 2]) * hz + 0.01f;
-      fits = fits && fabsf(mid) < 2048.f && ext < 100.f;  // (false for NaN)
+      const float ext = ax * hx + ay * hy + az * hz + 0.01f;
+      // Terms below 8192 in sum: five roundings of at most 2^-24 of it, here and in a sample's coordinate,
+      // stay under the margin.  (A brick one voxel thick bounds no term by its extent: a matrix whose
+      // large terms cancel would put its samples outside the box.  False for NaN.)
+      const float terms = ax * (fabsf(cu) + hx) + ay * (fabsf(cv) + hy) + az * (fabsf(cw) + hz) + fabsf(sh[i]) + (float)c;
+      fits = fits && terms < 8192.f && ext < 100.f;
       o[i] = fits ? (int)floorf(mid - ext) : 0;
       if (i == 0) o[i] &= ~(V - 1);
       len[i] = fits ? (int)floorf(mid + ext) + 2 - o[i] : 0;

@@ -129,3 +129,49 @@ def test_brick_edges_and_wide_matrices(built_lib, cuda, n, nw):
         for k in (0, 1):
             a, b = g[h][k].cpu().numpy(), o[h][k]
             assert np.abs(a - b).max() <= 2e-5 * np.abs(b).max(), (h, k)
+
+
+def test_cancelling_matrices_on_thin_bricks(built_lib, cuda):
+    """A box one voxel longer than whole bricks, with matrices whose entries are huge and cancel (or are
+    cancelled by the shift) at its far corner: the sums in different orders differ by whole voxels there,
+    so those samples do not come from the staged box.  The window's samples lie beyond it almost
+    everywhere; against a float32 restatement of the sampling in the kernel's order (FP32 products are
+    exact in float64, so one rounding each), whose coordinates must agree bit for bit."""
+    from emclarity_b200 import api
+    n, c = 17, 8
+    rng = np.random.default_rng(17)
+    vol = rng.standard_normal((n, n, n)).astype(np.float32)
+    cases = [(np.array([[1e7 + 3, -1e7, 0.3], [0, 1, 0], [0, 0, 1]]), (0, 0, 0)),
+             (np.array([[1, 0, 0], [0.25, 3e6, -3e6], [0, 0, 1]]), (0, -1.5, 0)),
+             (np.array([[1, 0, 0], [0, 1, 0], [0.3, 0.3, 2e6]]), (0, 0, -1.6e7)),
+             (np.eye(3), (0.5, 0.25, -0.75))]
+    mask = torch.ones((n, n, n), device="cuda")
+
+    def fma(a, b, d):  # one rounding: the product of two floats is exact in 64 bits, the sum nearly so
+        return (a.astype(np.float64) * b.astype(np.float64) + d.astype(np.float64)).astype(np.float32)
+
+    z, y, x = np.meshgrid(*[np.arange(n, dtype=np.float32) - c] * 3, indexing="ij")
+    for m, t in cases:
+        m32, t32 = m.astype(np.float32), np.asarray(t, np.float32)
+        s = []
+        for i in range(3):
+            v = fma(m32[i, 0:1], x, fma(m32[i, 1:2], y, (m32[i, 2] * z).astype(np.float32)))
+            s.append(((v + t32[i]).astype(np.float32) + np.float32(c)).astype(np.float64))
+        want = np.zeros((n, n, n))
+        for k in range(8):
+            o = (k & 1, (k >> 1) & 1, k >> 2)
+            w, ok, idx = 1.0, True, []
+            for a, oi in zip(s, o):
+                b = np.floor(a)
+                f = a - b
+                w = w * (f if oi else 1 - f)
+                ok = ok & (b + oi >= 0) & (b + oi < n)
+                idx.append(np.clip(b + oi, 0, n - 1).astype(int))
+            want += np.where(ok, w * vol[idx[2], idx[1], idx[0]], 0.0)
+        av = api.Average(mask)
+        kept = av.add(torch.from_numpy(vol)[None].cuda(), [m], [1], shifts=[t])
+        assert kept[0]
+        got = av.result(1)[0].cpu().numpy()
+        av.close()
+        want = (want - want.mean()) / want.std()
+        assert np.abs(got - want).max() <= 2e-5 * np.abs(want).max()
