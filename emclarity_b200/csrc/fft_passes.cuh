@@ -111,7 +111,9 @@ constexpr bool needs_smem_opt_in(size_t dynamic) { return dynamic + 1024 > 48 * 
 
 // ----------------------------------------------------------------- strided columns
 // Complex lines along a strided axis: element n of line (o, i) lives at
-// base + o*outer_pitch + i + n*stride, for i in [0, inner), o in [0, outer); in == out is allowed.
+// base + o*outer_pitch + i + n*stride, for i in [0, inner), o in [0, outer); in == out is allowed
+// (so neither pointer is restricted): a line's loads all precede its stores, by a barrier or, in
+// single-stage plans, in one thread.
 // A CTA transforms T consecutive lines (of the flattened (o, i), so that an inner extent that is no
 // multiple of T leaves no partial tiles) with J threads each, threads of a half-warp on consecutive
 // lines: the first stage takes its inputs from global memory, the last one stores its outputs there,
@@ -177,7 +179,7 @@ __device__ __forceinline__ void cols_stage(float2* line, int jt, bool active, co
 
 template <int L, int SIGN>
 __global__ void __launch_bounds__(ColsCfg<L>::T * ColsCfg<L>::J, ColsCfg<L>::min_blocks) k_cols(
-    const float2* __restrict__ in, float2* __restrict__ out, long stride, long inner, long lines, long outer_pitch,
+    const float2* in, float2* out, long stride, long inner, long lines, long outer_pitch,
     const float2* __restrict__ g_tw) {
   using C = ColsCfg<L>;
   extern __shared__ float2 smem[];

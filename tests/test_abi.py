@@ -100,3 +100,16 @@ def test_status_strings(built_lib):
     for s in (0, -1, -2, -3, -4, -5):
         assert built_lib.emc_status_string(s)
     assert b"sm_100a" in built_lib.emc_version()
+
+
+def test_kernels_launched_in_place_restrict_neither_pointer():
+    """The strided column transforms run with in == out (the y and z passes of every 3-D transform), so
+    their kernel may not promise the compiler that the two never alias."""
+    import os
+    import re
+    from emclarity_b200 import build
+    with open(os.path.join(build.CSRC, "fft_passes.cuh")) as f:
+        src = f.read()
+    sig = re.search(r"\bk_cols\((.*?)\)\s*\{", src, re.S).group(1)
+    data = [p.strip() for p in sig.split(",") if re.search(r"\b(in|out)$", p.strip())]
+    assert len(data) == 2 and not any("__restrict__" in p for p in data)
