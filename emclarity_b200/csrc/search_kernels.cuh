@@ -391,12 +391,24 @@ __global__ void __launch_bounds__(SearchCfg<N>::NT_A, SearchCfg<N>::MINB_A) k_se
   // shared-memory column of the y stages: kx = q, its mirror N - kx (N/2 for the packed column 0)
   const int mir = q == 0 ? Q : N - q;
   const int slot_k = (q & 7) * XA + (q >> 3) * XB, slot_m = (mir & 7) * XA + (mir >> 3) * XB;
-  float sum1 = 0.f, sum2 = 0.f;
-  // first x stage of a butterfly whose inputs lie in this thread's slots, in place
+  double sum1 = 0.0, sum2 = 0.0;
+  // First x stage of a butterfly whose inputs lie in this thread's slots, in place.  Without a weight on the
+  // reference its real-space sums are formed here, in FP64 from the samples on: E_R cancels for a
+  // reference with an offset (FP32 sums over a thread's samples put the CC at a mean of 100 sigma off by
+  // up to 6e-5, depending on the plane count; now 1e-7 at every count).  Here and not in the gather,
+  // whose registers are all taken; weighted searches skip it, unweighted ones take at most 3 % longer.
   auto first_x_stage = [&](float2* own) {
     float2 v[8];
 #pragma unroll
     for (int r = 0; r < 8; ++r) v[r] = own[r * XA];
+    if (!weighted) {
+#pragma unroll
+      for (int r = 0; r < 8; ++r) {
+        const double va = v[r].x, vb = v[r].y;
+        sum1 += va + vb;
+        sum2 = fma(va, va, fma(vb, vb, sum2));
+      }
+    }
     Dft<8, -1>::run(v);
 #pragma unroll
     for (int r = 0; r < 8; ++r) own[r * XA] = v[r];
@@ -475,10 +487,6 @@ __global__ void __launch_bounds__(SearchCfg<N>::NT_A, SearchCfg<N>::MINB_A) k_se
                 val[k] = ok[u][k] ? cell_trilinear(cv, f[u][k]) * mk[u][k] : 0.f;
               }
               own[u * XA] = make_float2(val[0], val[1]);
-              if (!weighted) {
-                sum1 += val[0] + val[1];
-                sum2 = fmaf(val[0], val[0], fmaf(val[1], val[1], sum2));
-              }
             }
           }
           first_x_stage(buf + j * XB + gq);
@@ -498,8 +506,6 @@ __global__ void __launch_bounds__(SearchCfg<N>::NT_A, SearchCfg<N>::MINB_A) k_se
               va *= __ldg(rf.mask + plane + (long)gq * N + x);
               vb *= __ldg(rf.mask + plane + (long)(gq + Q) * N + x);
             }
-            sum1 += va + vb;
-            sum2 = fmaf(va, va, fmaf(vb, vb, sum2));
             buf[r * XA + j * XB + gq] = make_float2(va, vb);
           }
           first_x_stage(buf + j * XB + gq);
@@ -579,8 +585,8 @@ __global__ void __launch_bounds__(SearchCfg<N>::NT_A, SearchCfg<N>::MINB_A) k_se
   if (!weighted) {
     // E_R from the real-space sums (Parseval) is needed only without a weight on the reference; with
     // one, pass B forms the weighted spectral energy (the branch is uniform over the block)
-    double t1 = block_sum((double)sum1, red[0]);
-    double t2 = block_sum((double)sum2, red[1]);
+    double t1 = block_sum(sum1, red[0]);
+    double t2 = block_sum(sum2, red[1]);
     if (threadIdx.x == 0) {
       atomicAdd(&a.stats[e].sum_r, t1);
       atomicAdd(&a.stats[e].sum_r2, t2);

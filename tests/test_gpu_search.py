@@ -5,6 +5,8 @@ Operands follow BH_multi_xcf_Translational_2.m:35-38 with BH_multi_xcf_Rotationa
 rotated reference (the search descriptor's `wedge`); the reference's weight refWdg multiplies the
 particle (folded into its spectrum; 1 unless a test sets it).  Every peak or best-orientation
 difference must be a near-tie in the oracle's own map (tests/searchcheck.py)."""
+import ctypes as C
+
 import numpy as np
 import pytest
 import torch
@@ -538,3 +540,44 @@ def test_unmasked_noise_reference_reaches_every_edge(built_lib, cuda, n, radius,
         check_cc_and_peaks(cc, pk, cc_o, pk_o, lambda o: O.xcf_translational(stored, P, mats[o], shift=sh, **kw)[2],
                            "n %d shift %s" % (n, sh))
     s.close()
+
+
+@pytest.mark.parametrize("n,planes", [(64, (1, 2, 4, 8)), (96, (1, 2, 4)), (128, (1, 2))])
+@pytest.mark.parametrize("interp", ["linear", "linear_border", "cubic"])
+def test_unweighted_energy_of_a_reference_with_an_offset(built_lib, cuda, n, planes, interp):
+    """Without a weight E_R = N^3 sum r^2 - (sum r)^2, which loses four digits for a mean of 100 standard
+    deviations: the sums have to be formed in 64 bits whatever the plane count.  The identity samples the
+    reference exactly, so against itself its CC is 1 but for the transforms' roundings, one of 2^-24 per
+    radix-2 level of N^3 points and four for the normalisation; FP32 sums over a thread's samples are off
+    by 2e-6 (four samples) to 3e-5 (128).  The allocation-free search takes the same sums."""
+    from emclarity_b200 import _lib as L
+    from emclarity_b200 import api
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    ref = torch.randn((n, n, n), device="cuda", generator=gen) + 100.0
+    q, e = api.particle_spectrum(ref)
+    tol = (3 * np.log2(n) + 4) * 2.0 ** -24
+    s = api.Search(peak_radius=2, interp=interp)
+    rid = s.add_reference(ref)
+    s.set_orientations(np.zeros((1, 3)))
+    cc = []
+    for p in planes:
+        s.set_planes(n, p)
+        c, pk, _ = s.run_host([s.particle(q, e.item(), rid, orient_count=1)])
+        assert np.array_equal(pk[0], [0, 0, 0])
+        cc.append(float(c[0]))
+    s.close()
+    assert np.abs(np.array(cc) - 1).max() <= tol, cc
+    assert max(cc) - min(cc) <= 2.0 ** -23, cc  # the plane count may move a rounding of the last bit
+    out = torch.zeros(1, device="cuda")
+    pk = torch.zeros((1, 3), dtype=torch.int32, device="cuda")
+    best = torch.zeros((1, 5), dtype=torch.int32, device="cuda")
+    zero = np.zeros(3)
+    eye = np.eye(3).flatten(order="F").copy()
+    pd = C.POINTER(C.c_double)
+    st = L.load().emc_search_plain_noalloc(
+        C.c_void_p(ref.data_ptr()), None, n, C.c_void_p(q.data_ptr()), e.item(), eye.ctypes.data_as(pd),
+        (C.c_float * 3)(0, 0, 0), zero.ctypes.data_as(pd), 1, 2, {"linear": 0, "cubic": 1, "linear_border": 2}[interp],
+        C.c_void_p(out.data_ptr()), C.c_void_p(pk.data_ptr()), C.c_void_p(best.data_ptr()),
+        C.c_void_p(torch.cuda.current_stream().cuda_stream))
+    assert st == 0
+    assert abs(out.item() - 1) <= tol
