@@ -697,7 +697,7 @@ __global__ void __launch_bounds__(SearchCfg<N>::NT_B, SearchCfg<N>::MINB_B) k_se
     loaded = it.particle;
     __syncthreads();
     // second stage, product, first inverse stage: kz = k1 + R2 k2 in registers
-    float ef = 0.f;  // |.|^2 of this thread's elements; the threads' sums are added in FP64
+    double ed = 0.0;  // |.|^2 of this thread's elements: a butterfly's eight in FP32, then FP64
     if (line) {
 #pragma unroll 1
       for (int k1 = jt; k1 < R2; k1 += JB) {
@@ -708,6 +708,7 @@ __global__ void __launch_bounds__(SearchCfg<N>::NT_B, SearchCfg<N>::MINB_B) k_se
 #pragma unroll
         for (int j = 1; j < 8; ++j) v[j] = cmul(v[j], s_tw[j * k1]);
         Dft<8, -1>::run(v);
+        float ef = 0.f;
 #pragma unroll
         for (int k2 = 0; k2 < 8; ++k2) {
           const bool origin = k1 + R2 * k2 + ky + kx == 0;
@@ -720,6 +721,7 @@ __global__ void __launch_bounds__(SearchCfg<N>::NT_B, SearchCfg<N>::MINB_B) k_se
           const float2 x = cmulc(qr[k2], r);
           v[k2] = origin ? make_float2(0.f, 0.f) : x;
         }
+        ed += (double)ef;
         if (!ONE && k1 + JB < R2) fetch(k1 + JB);
         Dft<8, 1>::run(v);
 #pragma unroll
@@ -729,7 +731,7 @@ __global__ void __launch_bounds__(SearchCfg<N>::NT_B, SearchCfg<N>::MINB_B) k_se
       }
     }
     if (weighted) {
-      const double t = block_sum(line ? hw * (double)ef : 0.0, red);  // (synchronises)
+      const double t = block_sum(line ? hw * ed : 0.0, red);  // (synchronises)
       if (threadIdx.x == 0) atomicAdd(&a.stats[e].energy_spec, t);
     } else {
       __syncthreads();
