@@ -81,9 +81,9 @@ constexpr int kPlaneOptions[] = {1, 2, 4, 8};
 template <int N, typename T>
 static emc_status set_attrs() {
   using C = SearchCfg<N>;
-  EMC_CUDA(cudaFuncSetAttribute(k_search_fwd_xy<N, T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  EMC_CUDA(cudaFuncSetAttribute(k_search_fwd_xy<N, T, kGatherCells>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)C::SMEM_A));
-  EMC_CUDA(cudaFuncSetAttribute(k_search_fwd_xy<N, T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  EMC_CUDA(cudaFuncSetAttribute(k_search_fwd_xy<N, T, kGatherCubic>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)C::SMEM_A));
   EMC_CUDA(cudaFuncSetAttribute(k_search_z_mul<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM_B));
   EMC_CUDA(cudaFuncSetAttribute(k_search_inv_peak<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM_C));
@@ -100,7 +100,7 @@ static emc_status launch_fwd(int g, const SearchChunkArgs& args, const float2* t
   SearchChunkArgs a = args;
   a.planes = g;
   // (every reference of a handle has its cells)
-  (a.interp == EMC_INTERP_CUBIC ? k_search_fwd_xy<N, T, false> : k_search_fwd_xy<N, T, true>)<<<
+  (a.interp == EMC_INTERP_CUBIC ? k_search_fwd_xy<N, T, kGatherCubic> : k_search_fwd_xy<N, T, kGatherCells>)<<<
       dim3(N / g, a.n_items), C::NT_A, C::SMEM_A, st>>>(a, tw);
   EMC_LAUNCH_CHECK();
   return EMC_OK;

@@ -224,6 +224,10 @@ __host__ __device__ constexpr bool planes_allowed(int N, int g) {
   return (g == 1 || g == 2 || g == 4 || g == 8) && g <= (N <= 64 ? 8 : N <= 96 ? 4 : 2);
 }
 
+// How pass A samples: the two trilinear modes through the cells, the same from the plain volume (a caller
+// without cells), or tricubic from the plain volume.
+enum Gather { kGatherCells, kGatherPlain, kGatherCubic };
+
 // The line transforms of passes A and B split N = 8 R2: with n = j + R2 r and k = k1 + 8 k2,
 //   X(k) = DFT_R2 over j of [ w_N^(j k1) DFT_8 over r of x(j + R2 r) ],
 // so a thread holds one 8-point or one R2-point butterfly of its own line, neighbouring threads hold
@@ -249,13 +253,13 @@ struct SearchCfg {
   static constexpr int JA = NT_A / Q;            // butterflies of a line formed side by side
   static_assert(NT_A % Q == 0 && R2 % JA == 0 && 8 % JA == 0 && JA % 4 == 0, "whole rounds and patches");
   static constexpr size_t SMEM_A = sizeof(float2) * (8 * (size_t)XA + N + N);
-  // resident pass-A CTAs asked of the compiler
-    // Cells in flight per thread (2 UNROLL_A) against resident warps: at 64^3 two and four CTAs per SM
-  // (1,095 ns per evaluation; four and three CTAs 1,150), at 96^3 and 128^3 four (3,490 and 9,180 ns;
-  // two: 3,760 and 10,760).  Four at one CTA more spill and lose by a third: local memory shares the
-  // L1 that the gather streams through.
+  // Resident pass-A CTAs asked of the compiler, and cells in flight per thread (2 UNROLL_A): at 64^3 two
+  // and four CTAs per SM (1,095 ns per evaluation; four and three CTAs 1,150), at 96^3 and 128^3 four
+  // (3,490 and 9,180 ns; two: 3,760 and 10,760).  Four at one CTA more spill and lose by a third: local
+  // memory shares the L1 that the gather streams through.  The tricubic sampler's 64 loads want more
+  // registers at 64^3 (64 masked orientations: 683 us at three CTAs, 715 at four, 731 at two).
   static constexpr int UNROLL_A = N == 64 ? 1 : 2;
-  static constexpr int MINB_A = N <= 96 ? 4 : 2;
+  static constexpr int min_blocks_a(Gather g) { return N > 96 ? 2 : N == 64 && g == kGatherCubic ? 3 : 4; }
   // ---- pass B: the z lines of one ky, the R2-point stage first (its inputs come straight from global
   // memory) and the 8-point one second, so that the product needs 8 spectrum and weight elements per
   // butterfly.  S1 rows hold column N/2 first, then 0 .. N/2-1, padded to whole 32-byte sectors;
@@ -334,14 +338,17 @@ __device__ __forceinline__ float cell_trilinear(const float v[8], const float f[
   return fmaf(f[2], c1 - c0, c0);
 }
 
-// Sampling point of voxel (x, y, z) under the matrix rows m, and the reference's value there, for
-// the modes without cells.
-template <typename T>
-__device__ __noinline__ float sample_any(int mode, const T* __restrict__ src, int n, const float* __restrict__ m,
-                                         float u, float v, float w) {
+// The reference's value at the sampling point of voxel (u, v, w) (from the centre) under the matrix rows m,
+// for the modes without cells.
+template <Gather GATHER, typename T>
+__device__ __forceinline__ float sample_plain(int mode, const T* __restrict__ src, int n, const float* __restrict__ m,
+                                              float u, float v, float w) {
   const float c = (float)(n / 2);
-  return sample(mode, src, n, n, n, fmaf(m[0], u, fmaf(m[1], v, m[2] * w)) + c,
-                fmaf(m[3], u, fmaf(m[4], v, m[5] * w)) + c, fmaf(m[6], u, fmaf(m[7], v, m[8] * w)) + c);
+  const float sx = fmaf(m[0], u, fmaf(m[1], v, m[2] * w)) + c, sy = fmaf(m[3], u, fmaf(m[4], v, m[5] * w)) + c,
+              sz = fmaf(m[6], u, fmaf(m[7], v, m[8] * w)) + c;
+  return GATHER == kGatherCubic ? sample_cubic(src, n, n, n, sx, sy, sz)
+         : mode == EMC_INTERP_LINEAR_BORDER ? sample_linear_border(src, n, n, n, sx, sy, sz)
+                                            : sample_linear(src, n, n, n, sx, sy, sz);
 }
 
 // ------------------------------------------------------------------ pass A
@@ -350,10 +357,9 @@ __device__ __noinline__ float sample_any(int mode, const T* __restrict__ src, in
 // memory only in the thread's own slots.  A warp takes 8 rows x 4 columns of the plane and reads the
 // cells from bricks (see brick_index); floors by a round-down addition (kFloorMagic).
 //
-// CELLS: the two trilinear modes through the cells; else any mode from the plain volume (tricubic, or
-// a caller without cells), its sampler a call.
-template <int N, typename T, bool CELLS>
-__global__ void __launch_bounds__(SearchCfg<N>::NT_A, SearchCfg<N>::MINB_A) k_search_fwd_xy(
+// GATHER: see Gather.
+template <int N, typename T, Gather GATHER>
+__global__ void __launch_bounds__(SearchCfg<N>::NT_A, SearchCfg<N>::min_blocks_a(GATHER)) k_search_fwd_xy(
     const SearchChunkArgs a, const float2* __restrict__ g_tw) {
   using C = SearchCfg<N>;
   constexpr int R2 = C::R2, Q = C::Q, XA = C::XA, XB = C::XB, JA = C::JA;
@@ -422,7 +428,7 @@ __global__ void __launch_bounds__(SearchCfg<N>::NT_A, SearchCfg<N>::MINB_A) k_se
       const int gq = (lane & 7) + 8 * (warp % (Q / 8)), gj = (lane >> 3) + 4 * (warp / (Q / 8));
       const float tx = pt.shift[0], pw = (float)(z - c) - pt.shift[2];
       const float pva = (float)(gq - c) - pt.shift[1], pvb = (float)(gq + Q - c) - pt.shift[1];
-      if constexpr (CELLS) {
+      if constexpr (GATHER == kGatherCells) {
         constexpr int U = C::UNROLL_A;
         float base[2][3], mx[3];  // sample points at u = 0 of the two rows
 #pragma unroll
@@ -492,24 +498,20 @@ __global__ void __launch_bounds__(SearchCfg<N>::NT_A, SearchCfg<N>::MINB_A) k_se
           first_x_stage(buf + j * XB + gq);
         }
       } else {
+        // 32 consecutive voxels of a row per warp: the plain volume is x fastest, so their loads share lines
+        // where the patches' rows do not.  (64 tricubic orientations near the identity: 64^3 1,039 -> 683 us,
+        // 96^3 3,588 -> 2,824, 128^3 9,196 -> 5,945 against one call of the sampler per voxel of a patch.)
         const T* src = reinterpret_cast<const T*>(rf.data);
-        const long plane = (long)z * N * N;
-#pragma unroll 1
-        for (int j = gj; j < R2; j += JA) {
-#pragma unroll 1
-          for (int r = 0; r < 8; ++r) {
-            const int x = j + R2 * r;
-            const float pu = (float)(x - c) - tx;
-            float va = sample_any(a.interp, src, N, s_m, pu, pva, pw);
-            float vb = sample_any(a.interp, src, N, s_m, pu, pvb, pw);
-            if (rf.mask) {
-              va *= __ldg(rf.mask + plane + (long)gq * N + x);
-              vb *= __ldg(rf.mask + plane + (long)(gq + Q) * N + x);
-            }
-            buf[r * XA + j * XB + gq] = make_float2(va, vb);
-          }
-          first_x_stage(buf + j * XB + gq);
+        const float* mask = rf.mask ? rf.mask + (long)z * N * N : nullptr;
+        for (int i = threadIdx.x; i < N * N; i += C::NT_A) {
+          const int x = i % N, y = i / N;
+          float v = sample_plain<GATHER>(a.interp, src, N, s_m, (float)(x - c) - tx, (float)(y - c) - pt.shift[1], pw);
+          if (mask) v *= __ldg(mask + i);
+          reinterpret_cast<float*>(buf + (x / R2) * XA + (x % R2) * XB + y % Q)[y / Q] = v;
         }
+        __syncthreads();
+#pragma unroll 1
+        for (int j = gj; j < R2; j += JA) first_x_stage(buf + j * XB + gq);
       }
     }
     __syncthreads();

@@ -115,7 +115,10 @@ __global__ void k_noalloc_outputs(const NoallocResult* __restrict__ res, int n_o
 template <int N, typename T>
 emc_status set_attrs_noalloc() {
   using C = SearchCfg<N>;
-  EMC_CUDA(cudaFuncSetAttribute(k_search_fwd_xy<N, T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM_A));
+  EMC_CUDA(cudaFuncSetAttribute(k_search_fwd_xy<N, T, kGatherPlain>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)C::SMEM_A));
+  EMC_CUDA(cudaFuncSetAttribute(k_search_fwd_xy<N, T, kGatherCubic>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)C::SMEM_A));
   EMC_CUDA(cudaFuncSetAttribute(k_search_z_mul<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM_B));
   EMC_CUDA(cudaFuncSetAttribute(k_search_inv_peak<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM_C));
   return EMC_OK;
@@ -166,7 +169,8 @@ emc_status run_chunks(const SearchChunkArgs& proto, int n_orient, int chunk, con
     EMC_CUDA(cudaMemsetAsync(a.stats, 0, sizeof(EvalStats) * a.n_items, st));
     EMC_CUDA(cudaMemsetAsync(a.keys, 0, sizeof(unsigned long long) * a.n_items, st));
     a.planes = 1;
-    k_search_fwd_xy<N, float, false><<<dim3(N, a.n_items), C::NT_A, C::SMEM_A, st>>>(a, tw);
+    (a.interp == EMC_INTERP_CUBIC ? k_search_fwd_xy<N, float, kGatherCubic> : k_search_fwd_xy<N, float, kGatherPlain>)<<<
+        dim3(N, a.n_items), C::NT_A, C::SMEM_A, st>>>(a, tw);
     k_search_z_mul<N><<<dim3(N, (a.n_items + C::EVALS_B - 1) / C::EVALS_B), C::NT_B, C::SMEM_B, st>>>(a, tw);
     k_search_inv_peak<N><<<dim3(w, a.n_items), C::NT_BC, C::SMEM_C, st>>>(a, tw);
     k_noalloc_decode<<<(a.n_items + 127) / 128, 128, 0, st>>>(a, N, res, best);

@@ -581,3 +581,28 @@ def test_unweighted_energy_of_a_reference_with_an_offset(built_lib, cuda, n, pla
         C.c_void_p(torch.cuda.current_stream().cuda_stream))
     assert st == 0
     assert abs(out.item() - 1) <= tol
+
+
+@pytest.mark.parametrize("n,store", [(64, "bf16"), (96, "f32"), (96, "bf16"), (128, "f32")])
+def test_tricubic_search_at_every_box_matches_oracle(built_lib, cuda, n, store):
+    """The tricubic sampler's gather (whole rows from the plain volume) over a noise reference up to its
+    faces, masked, with a shift; tolerance as everywhere."""
+    from emclarity_b200 import api, synthetic
+    rng = np.random.default_rng(5 * n)
+    ref = rng.standard_normal((n, n, n)).astype(np.float32)
+    mask = synthetic.soft_sphere_mask(n, 28 * n / 64)
+    P, _ = O.particle_spectrum(rng.standard_normal((n, n, n)).astype(np.float32))
+    q = torch.from_numpy(P.astype(np.complex64)).cuda()
+    energy = float(np.sum(np.abs(P) ** 2 * np.where(np.arange(n // 2 + 1) % (n // 2) == 0, 1.0, 2.0)))
+    grid = np.array([[0.0, 0.0, 0.0], [25.0, 50.0, -70.0]])
+    shift = (1.5, -2.25, 0.75)
+    s = api.Search(peak_radius=5, interp="cubic")
+    rid = s.add_reference(torch.from_numpy(ref).cuda(), torch.from_numpy(mask).cuda(), store=store)
+    s.set_orientations(grid)
+    cc, pk, _ = s.run_host([s.particle(q, energy, rid, shift=shift, orient_count=len(grid))])
+    s.close()
+    stored = torch.from_numpy(ref).bfloat16().float().numpy() if store == "bf16" else ref
+    kw = dict(interp=1, mask=mask, shift=shift)
+    mats = api.search_matrices(grid)
+    cc_o, pk_o = O.search(stored, P, mats, radius=5, **kw)
+    check_cc_and_peaks(cc, pk, cc_o, pk_o, lambda o: O.xcf_translational(stored, P, mats[o], **kw)[2], "n %d" % n)
