@@ -283,7 +283,10 @@ EMC_API emc_status emc_search_create(emc_search_t* out);
 /* Registers a reference volume (n^3 floats, device), an optional real-space mask
  * applied after rotation (n^3, or NULL) and an optional real half-spectrum weight
  * applied to the rotated reference's spectrum (bandpass; NULL = 1).  store_dtype:
- * EMC_DTYPE_F32 or EMC_DTYPE_BF16 (mixed precision: interpolation stays FP32). */
+ * EMC_DTYPE_F32 or EMC_DTYPE_BF16 (mixed precision: interpolation stays FP32).
+ * The handle keeps the volume, its trilinear corner cells in two orders (rows for the adjoint, bricks
+ * for the search) and the mask in two: 21 / 70 / 164 MB for a masked FP32 reference of 64^3 / 96^3 /
+ * 128^3, 12 / 38 / 90 MB in BF16. */
 EMC_API emc_status emc_search_add_reference(emc_search_t s, const float* d_ref, int n,
                                     const float* d_mask, const float* d_wref,
                                     int store_dtype, int* ref_id, void* stream);
