@@ -89,11 +89,7 @@ struct SfTilt {
   float occ, expo;
 };
 
-__global__ void k_sf3d_tables(const SfTilt* __restrict__ tilts, int nx, int ny, float4* __restrict__ tab) {
-  const int y = blockIdx.x * blockDim.x + threadIdx.x;
-  const int x = blockIdx.y * blockDim.y + threadIdx.y;
-  if (x >= nx || y >= ny) return;
-  const SfTilt t = tilts[blockIdx.z];
+__device__ __forceinline__ float4 sf_pixel(const SfTilt& t, int x, int y) {
   const int xs = x - t.g.ox, ys = y - t.g.oy;
   const float fy = (float)ys * t.g.fvy;
   const float fx = (float)xs * t.g.fvx;
@@ -101,12 +97,21 @@ __global__ void k_sf3d_tables(const SfTilt* __restrict__ tilts, int nx, int ny, 
   const float r2 = fx * fx + fy * fy;
   const float rw = t.occ * (xs == 0 ? 0.2f : fabsf((float)xs));
   float4 v;
-  v.x = t.c.cs_term * (r2 * r2);
-  v.y = t.c.df_term * r2;
+  // (products rounded on their own, as when they pass through the table)
+  v.x = __fmul_rn(t.c.cs_term, r2 * r2);
+  v.y = __fmul_rn(t.c.df_term, r2);
   v.z = cosf(2.0f * (phi - t.c.ast));
   // Grant-Grigorieff critical exposure as in k_ctf2d
-  v.w = rw * expf((-0.5f * t.expo) / (0.24499f * powf(r2, -0.8325f) + 2.81410f));
-  tab[((long)blockIdx.z * nx + x) * ny + y] = v;
+  v.w = __fmul_rn(rw, expf((-0.5f * t.expo) / (0.24499f * powf(r2, -0.8325f) + 2.81410f)));
+  return v;
+}
+
+__global__ void k_sf3d_tables(const SfTilt* __restrict__ tilts, int nx, int ny, float4* __restrict__ tab) {
+  const int y = blockIdx.x * blockDim.x + threadIdx.x;
+  const int x = blockIdx.y * blockDim.y + threadIdx.y;
+  if (x >= nx || y >= ny) return;
+  const SfTilt t = tilts[blockIdx.z];
+  tab[((long)blockIdx.z * nx + x) * ny + y] = sf_pixel(t, x, y);
 }
 
 // Volumes whose image values lie together: K = 4 (a 16-byte load serves four volumes), or 1 for a
@@ -146,7 +151,9 @@ struct SfVols<1> {
 // The tilt images of `count` volumes, [group of K volumes][tilt][x][y][volume] and one column of zeros
 // after each group (lanes along y, as k_sf3d_volumes reads them).  A thread keeps its pixel's table
 // entry and walks the groups: the radius, the angle and the exposure filter, most of an image's
-// arithmetic, are formed once per pixel instead of per volume.
+// arithmetic, are formed once per pixel instead of per volume.  Without a table (K = 1) it forms the entry
+// itself, once per volume: the table would be four fifths of the scratch (one volume of 1024 x 1024 x 16:
+// 4,146 -> 976 us without it, most of the difference mapping memory).
 template <int K>
 __global__ void __launch_bounds__(256) k_sf3d_images(const float4* __restrict__ tab, const SfTilt* __restrict__ tilts,
                                                      const float2* __restrict__ df, int ntilts, long npix, int ny,
@@ -154,7 +161,7 @@ __global__ void __launch_bounds__(256) k_sf3d_images(const float4* __restrict__ 
   const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
   const int t = blockIdx.y;
   if (i >= npix) return;
-  const float4 v = tab[(long)t * npix + i];
+  const float4 v = K == 1 ? sf_pixel(tilts[t], (int)(i / ny), (int)(i % ny)) : tab[(long)t * npix + i];
   const float amp = tilts[t].c.amp_phase;
   const long ngroup = npix * ntilts + ny;
   for (int g = blockIdx.z; g * K < count; g += gridDim.z) {
@@ -389,7 +396,7 @@ static emc_status sf3d_batch(const std::vector<SfTilt>& ts, const std::vector<fl
   const int chunk = (int)std::max<size_t>(1, std::min<size_t>({(size_t)ngroups, (size_t)(48ull << 20) / group, 65535}));
   auto up = [](size_t b) { return (b + 255) / 256 * 256; };
   const size_t t_bytes = up(sizeof(SfTilt) * n), d_bytes = up(sizeof(float2) * df.size());
-  const size_t k_bytes = up(sizeof(unsigned) * count), tab_bytes = up(sizeof(float4) * (size_t)n * npix);
+  const size_t k_bytes = up(sizeof(unsigned) * count), tab_bytes = K == 1 ? 0 : up(sizeof(float4) * (size_t)n * npix);
   std::vector<char> host(t_bytes + d_bytes);
   memcpy(host.data(), ts.data(), sizeof(SfTilt) * n);
   memcpy(host.data() + t_bytes, df.data(), sizeof(float2) * df.size());
@@ -402,7 +409,7 @@ static emc_status sf3d_batch(const std::vector<SfTilt>& ts, const std::vector<fl
   Px* imgs = reinterpret_cast<Px*>(buf + t_bytes + d_bytes + k_bytes + tab_bytes);
   cudaError_t e = cudaMemcpyAsync(buf, host.data(), host.size(), cudaMemcpyHostToDevice, st);
   if (e == cudaSuccess && shifted) e = cudaMemsetAsync(keys, 0xff, sizeof(unsigned) * count, st);
-  if (e == cudaSuccess) {
+  if (e == cudaSuccess && K > 1) {
     k_sf3d_tables<<<dim3((ny + 31) / 32, (nx + 7) / 8, n), dim3(32, 8), 0, st>>>(d_t, nx, ny, tab);
     e = cudaGetLastError();
   }
@@ -586,8 +593,13 @@ emc_status emc_sf3d_particles(const unsigned size[3], double sampling, const dou
       df[(size_t)p * n + r] = make_float2(0.5f * (d1 + d2), 0.5f * (d1 - d2));
     }
   }
-  return (count > 1 ? emc::sf3d_batch<4> : emc::sf3d_batch<1>)(ts, df, count, nx, ny, nz, 1, true, d_out,
-                                                                emc::as_stream(stream));
+  // Groups of four share a table: 32 bytes of scratch per pixel and tilt.  Past 128 MiB of that (41 tilts
+  // above 320^2) volumes go one at a time, with 4 bytes: mapping the scratch then costs more than the
+  // groups save (41 tilts, two volumes of 800 x 800 x 4: 1,052 us against 3,984; three of 512 x 512 x 16: 823
+  // against 1,860), and the call stays within the memory that it took without groups.
+  const bool groups = count > 1 && 32 * (size_t)n * nx * ny <= (128ull << 20);
+  return (groups ? emc::sf3d_batch<4> : emc::sf3d_batch<1>)(ts, df, count, nx, ny, nz, 1, true, d_out,
+                                                            emc::as_stream(stream));
 }
 
 }  // extern "C"

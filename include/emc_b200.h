@@ -141,7 +141,8 @@ EMC_API emc_status emc_ctf2d_exposure(const emc_ctf_params* p, int nx, int ny, i
  *         nTilts, tilt[n], exposure[n], occupancy[n]) (mexFiles/mexSF3D.cu:84-302):
  * sum over tilts of the exposure-weighted CTF^2 inserted on the tilted central
  * slab.  Host arrays of n_tilts entries; d_out: size[0]*size[1]*size[2] floats,
- * overwritten.  half must be 0 (the reference only builds the full grid). */
+ * overwritten.  half must be 0 (the reference only builds the full grid).  Scratch: 4 bytes per
+ * image pixel and tilt; synchronises the stream. */
 EMC_API emc_status emc_sf3d(int half, int squared, const unsigned size[3], const float* pix,
                     const float* wavelength, const float* cs_mm, const float* df1,
                     const float* df2, const float* astig_deg, const float* amp_contrast,
@@ -517,9 +518,11 @@ EMC_API emc_status emc_centred_to_half(const float* d_in, int nx, int ny, int nz
  * :16-30) is sorted on column 1 and cast to single; each particle's defocus is offset by the
  * height of its position along every tilt's beam; the volumes come from emc_sf3d (full grid, CTF
  * squared) and are shifted by -(min - 1e-4).  xyz: [count][3]; recon_geometry: the 2 x 3
- * reconGeometry, row-major (size, then shift); d_out: [count][size^3].  The tilt
- * images are made by one launch per chunk of particles (about 48 MiB of images) and accumulated by
- * a second; the call synchronises the stream once. */
+ * reconGeometry, row-major (size, then shift); d_out: [count][size^3].  The tilt images are made by
+ * one launch per chunk of particles and accumulated by a second.  Scratch: 16 bytes per image pixel
+ * and tilt for a table and up to 48 MiB of images (at least those of one group of four particles, 16
+ * bytes per pixel and tilt); past 128 MiB of the two, 48 MiB of images (at least one particle's, 4
+ * bytes).  The call synchronises the stream once. */
 EMC_API emc_status emc_sf3d_particles(const unsigned size[3], double sampling, const double* tlt, int rows,
                                       int cols, const double* xyz, const double recon_geometry[6], int count,
                                       float* d_out, void* stream);

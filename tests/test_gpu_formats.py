@@ -156,3 +156,35 @@ def test_sf3d_particles_several_groups_per_list(built_lib, cuda, ny, tilts):
     ref = O.sf3d_particles_np(size, 2.0, t, xyz[pick], rg)
     for p, r in zip(pick, ref):
         assert np.abs(got[p] - r).max() <= 2e-4 * np.abs(r).max(), (p, np.abs(got[p] - r).max())
+
+
+def _scratch_high(call):
+    """Bytes that a call held at most from the device's stream-ordered pool."""
+    rt = pytest.importorskip("cuda.bindings.runtime")
+    driver = pytest.importorskip("cuda.bindings.driver")
+    torch.cuda.synchronize()
+    err, pool = rt.cudaDeviceGetDefaultMemPool(torch.cuda.current_device())
+    assert err == rt.cudaError_t.cudaSuccess
+    high = rt.cudaMemPoolAttr.cudaMemPoolAttrUsedMemHigh
+    rt.cudaMemPoolSetAttribute(pool, high, driver.cuuint64_t(0))
+    before = int(rt.cudaMemPoolGetAttribute(pool, rt.cudaMemPoolAttr.cudaMemPoolAttrUsedMemCurrent)[1])
+    out = call()
+    torch.cuda.synchronize()
+    return int(rt.cudaMemPoolGetAttribute(pool, high)[1]) - before, out
+
+
+@pytest.mark.parametrize("count", [1, 2])
+def test_sf3d_scratch_of_wide_images(built_lib, cuda, count):
+    """Wide images go one volume at a time without a table: 4 bytes of scratch per pixel and tilt (and a
+    MiB for the tilts, the zero columns and rounding), same values as the oracle's."""
+    from emclarity_b200 import api
+    rng = np.random.default_rng(count)
+    tilts, size = 41, (512, 330, 2)
+    t = _tilt_table(rng, tilts)
+    rg = np.array([[512, 512, 256], [0.0, 1.0, -2.0]])
+    xyz = rng.uniform(1, [512, 512, 256], (count, 3))
+    used, got = _scratch_high(lambda: api.sf3d_particles(size, 2.0, t, xyz, rg))
+    assert used <= 4 * tilts * size[0] * size[1] * max(1, (48 << 20) // (4 * tilts * size[0] * size[1])) + (1 << 20)
+    ref = O.sf3d_particles_np(size, 2.0, t, xyz, rg)
+    for g, r in zip(got.cpu().numpy(), ref):
+        assert np.abs(g - r).max() <= 2e-4 * np.abs(r).max(), np.abs(g - r).max()
