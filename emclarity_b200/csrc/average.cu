@@ -115,7 +115,9 @@ __device__ __forceinline__ void zero_piece(float* p) {
 // (8-way conflicts, 2.68 ms); conversion instructions and one sample at a time cost 3.10 ms.
 // V: voxels per copy, 4 / 2 / 1 as the edge and the base alignment allow.  A matrix that is no
 // rotation can need a larger box than the staging holds; such a brick samples global memory.
-constexpr int kBrickXY = 16, kBrickZ = 8;
+// V = 0: bricks 2 deep that sample global memory, for launches of so few CTAs that the copies, one operator
+// after another, are a chain of latencies and not a saving (see launch_rotate).
+constexpr int kBrickXY = 16, kBrickZ = 8, kThinZ = 2;
 // A rotated brick's box spans at most 2 |(7.5, 7.5, 3.5)| = 22.3 voxels along any axis; one more for
 // the upper corners, one for the fraction, and up to three to start x on a copy boundary.
 constexpr int kBoxYZ = 26, kBoxX = 28;
@@ -158,7 +160,7 @@ __device__ __forceinline__ unsigned long long avg_sample_staged2(const float* __
   return acc;
 }
 
-template <int V>
+template <int V, int Z>
 __global__ void __launch_bounds__(256, 3) k_avg_rotate(const float* __restrict__ vols, long vol_stride,
                                                     const int* __restrict__ vol_index, int n,
                                                     const float* __restrict__ mats,
@@ -175,9 +177,9 @@ __global__ void __launch_bounds__(256, 3) k_avg_rotate(const float* __restrict__
   const int nbx = (n + kBrickXY - 1) / kBrickXY;
   const int b = blockIdx.x;
   const int t = threadIdx.x;
-  const int bx = (b % nbx) * kBrickXY, by = ((b / nbx) % nbx) * kBrickXY, bz = (b / (nbx * nbx)) * kBrickZ;
+  const int bx = (b % nbx) * kBrickXY, by = ((b / nbx) % nbx) * kBrickXY, bz = (b / (nbx * nbx)) * Z;
   const int x = bx + t % kBrickXY, y = by + t / kBrickXY;
-  const int nz = min(kBrickZ, n - bz);
+  const int nz = min(Z, n - bz);
   const bool in_xy = x < n && y < n;
   const int c = n / 2;
   const float zero[3] = {0.f, 0.f, 0.f};
@@ -185,99 +187,104 @@ __global__ void __launch_bounds__(256, 3) k_avg_rotate(const float* __restrict__
   const float* src = vols + (long)(vi < 0 ? 0 : vi) * vol_stride;
   const float* m0 = mats + (long)p * kAvgMaxSym * 9;
   const float u = (float)(x - c), v = (float)(y - c);
-  float acc[kBrickZ];
+  float acc[Z];
 #pragma unroll
-  for (int q = 0; q < kBrickZ; ++q) acc[q] = 0.f;
+  for (int q = 0; q < Z; ++q) acc[q] = 0.f;
   for (int k = 0; k < (vi < 0 ? 0 : pr.nsym); ++k) {
     const float* m = m0 + 9 * k;
-    // the box of the brick's samples: centre and half extent along each axis, a margin for rounding
-    const float hx = 0.5f * (float)(min(kBrickXY, n - bx) - 1), hy = 0.5f * (float)(min(kBrickXY, n - by) - 1),
-                hz = 0.5f * (float)(nz - 1);
-    const float cu = (float)(bx - c) + hx, cv = (float)(by - c) + hy, cw = (float)(bz - c) + hz;
-    int o[3], len[3];
-    bool fits = true;
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-      const float ax = fabsf(m[3 * i]), ay = fabsf(m[3 * i + 1]), az = fabsf(m[3 * i + 2]);
-      const float mid = m[3 * i] * cu + m[3 * i + 1] * cv + m[3 * i + 2] * cw + sh[i] + (float)c;
-      const float ext = ax * hx + ay * hy + az * hz + 0.01f;
-      // Terms below 8192 in sum: five roundings of at most 2^-24 of it, here and in a sample's coordinate,
-      // stay under the margin.  (A brick one voxel thick bounds no term by its extent: a matrix whose
-      // large terms cancel would put its samples outside the box.  False for NaN.)
-      const float terms = ax * (fabsf(cu) + hx) + ay * (fabsf(cv) + hy) + az * (fabsf(cw) + hz) + fabsf(sh[i]) + (float)c;
-      fits = fits && terms < 8192.f && ext < 100.f;
-      o[i] = fits ? (int)floorf(mid - ext) : 0;
-      if (i == 0) o[i] &= ~(V - 1);
-      len[i] = fits ? (int)floorf(mid + ext) + 2 - o[i] : 0;
-    }
-    len[0] = (len[0] + V - 1) / V * V;
-    fits = fits && len[0] <= kBoxX && len[1] <= kBoxYZ && len[2] <= kBoxYZ;  // the same for the whole CTA
-    if (fits) {
-      if (k > 0) __syncthreads();  // the previous operator's samples have been formed
-      // thread t copies pieces t % 8, + 8, .. of row t / 8 (of at most 26) in every plane
-      const int yy = t >> 3, gy = o[1] + yy, pieces = len[0] / V;
-      if (yy < len[1]) {
-        const bool in_y = gy >= 0 && gy < n;
-#pragma unroll
-        for (int w0 = 0; w0 < kBoxX / V; w0 += 8) {
-          const int w = w0 + (t & 7), gx = o[0] + w * V;
-          if (w < pieces) {
-            float* to = s_box + yy * kBoxX + w * V;
-            // planes [za, zb) of this piece lie in the volume, the others are zeros
-            const bool in = in_y && gx >= 0 && gx < n;
-            const int za = in ? max(0, min(-o[2], len[2])) : len[2], zb = in ? max(za, min(n - o[2], len[2])) : len[2];
-            const float* from = src + (in && za < zb ? ((long)(o[2] + za) * n + gy) * n + gx : 0);
-#pragma unroll 4
-            for (int zz = za; zz < zb; ++zz) {
-              cp_async<4 * V>(to + zz * (kBoxYZ * kBoxX), from);
-              from += (long)n * n;
-            }
-            for (int zz = 0; zz < za; ++zz) zero_piece<V>(to + zz * (kBoxYZ * kBoxX));
-            for (int zz = zb; zz < len[2]; ++zz) zero_piece<V>(to + zz * (kBoxYZ * kBoxX));
-          }
-        }
-      }
-      cp_async_commit();
-      cp_async_wait<0>();
-      __syncthreads();
-    }
-    const unsigned base = 0u - (((unsigned)o[2] + kFloorBits) * (unsigned)(kBoxYZ * kBoxX) +
-                                ((unsigned)o[1] + kFloorBits) * (unsigned)kBoxX + (unsigned)o[0] + kFloorBits);
-    if (in_xy && fits) {
-      // s = M u, + t, + c: the operations of avg_sample, two planes at a time.  (With the last plane of
-      // an odd count its pair repeats it.)
-      unsigned long long mz[3], ts[3];
-      const unsigned long long uu = pack2(u, u), vv = pack2(v, v), cc = pack2((float)c, (float)c);
+    bool staged = false;
+    if constexpr (V > 0) {
+      // the box of the brick's samples: centre and half extent along each axis, a margin for rounding
+      const float hx = 0.5f * (float)(min(kBrickXY, n - bx) - 1), hy = 0.5f * (float)(min(kBrickXY, n - by) - 1),
+                  hz = 0.5f * (float)(nz - 1);
+      const float cu = (float)(bx - c) + hx, cv = (float)(by - c) + hy, cw = (float)(bz - c) + hz;
+      int o[3], len[3];
+      bool fits = true;
 #pragma unroll
       for (int i = 0; i < 3; ++i) {
-        mz[i] = pack2(m[3 * i + 2], m[3 * i + 2]);
-        ts[i] = pack2(sh[i], sh[i]);
+        const float ax = fabsf(m[3 * i]), ay = fabsf(m[3 * i + 1]), az = fabsf(m[3 * i + 2]);
+        const float mid = m[3 * i] * cu + m[3 * i + 1] * cv + m[3 * i + 2] * cw + sh[i] + (float)c;
+        const float ext = ax * hx + ay * hy + az * hz + 0.01f;
+        // Terms below 8192 in sum: five roundings of at most 2^-24 of it, here and in a sample's coordinate,
+        // stay under the margin.  (A brick one voxel thick bounds no term by its extent: a matrix whose
+        // large terms cancel would put its samples outside the box.  False for NaN.)
+        const float terms = ax * (fabsf(cu) + hx) + ay * (fabsf(cv) + hy) + az * (fabsf(cw) + hz) + fabsf(sh[i]) + (float)c;
+        fits = fits && terms < 8192.f && ext < 100.f;
+        o[i] = fits ? (int)floorf(mid - ext) : 0;
+        if (i == 0) o[i] &= ~(V - 1);
+        len[i] = fits ? (int)floorf(mid + ext) + 2 - o[i] : 0;
       }
+      len[0] = (len[0] + V - 1) / V * V;
+      fits = fits && len[0] <= kBoxX && len[1] <= kBoxYZ && len[2] <= kBoxYZ;  // the same for the whole CTA
+      if (fits) {
+        if (k > 0) __syncthreads();  // the previous operator's samples have been formed
+        // thread t copies pieces t % 8, + 8, .. of row t / 8 (of at most 26) in every plane
+        const int yy = t >> 3, gy = o[1] + yy, pieces = len[0] / V;
+        if (yy < len[1]) {
+          const bool in_y = gy >= 0 && gy < n;
 #pragma unroll
-      for (int q = 0; q < kBrickZ; q += 2) {
-        if (q < nz) {
-          const unsigned long long ww = pack2((float)(bz + q - c), (float)(bz + min(q + 1, nz - 1) - c));
-          unsigned long long sp[3];
-#pragma unroll
-          for (int i = 0; i < 3; ++i) {
-            const unsigned long long a0 = pack2(m[3 * i], m[3 * i]), a1 = pack2(m[3 * i + 1], m[3 * i + 1]);
-            sp[i] = fadd2(fadd2(ffma2(a0, uu, ffma2(a1, vv, fmul2(mz[i], ww))), ts[i]), cc);
+          for (int w0 = 0; w0 < kBoxX / V; w0 += 8) {
+            const int w = w0 + (t & 7), gx = o[0] + w * V;
+            if (w < pieces) {
+              float* to = s_box + yy * kBoxX + w * V;
+              // planes [za, zb) of this piece lie in the volume, the others are zeros
+              const bool in = in_y && gx >= 0 && gx < n;
+              const int za = in ? max(0, min(-o[2], len[2])) : len[2], zb = in ? max(za, min(n - o[2], len[2])) : len[2];
+              const float* from = src + (in && za < zb ? ((long)(o[2] + za) * n + gy) * n + gx : 0);
+#pragma unroll 4
+              for (int zz = za; zz < zb; ++zz) {
+                cp_async<4 * V>(to + zz * (kBoxYZ * kBoxX), from);
+                from += (long)n * n;
+              }
+              for (int zz = 0; zz < za; ++zz) zero_piece<V>(to + zz * (kBoxYZ * kBoxX));
+              for (int zz = zb; zz < len[2]; ++zz) zero_piece<V>(to + zz * (kBoxYZ * kBoxX));
+            }
           }
-          const float2 val = unpack2(avg_sample_staged2(s_box, base, sp));
-          acc[q] += val.x;
-          acc[q + 1] += val.y;
+        }
+        cp_async_commit();
+        cp_async_wait<0>();
+        __syncthreads();
+      }
+      const unsigned base = 0u - (((unsigned)o[2] + kFloorBits) * (unsigned)(kBoxYZ * kBoxX) +
+                                  ((unsigned)o[1] + kFloorBits) * (unsigned)kBoxX + (unsigned)o[0] + kFloorBits);
+      if (in_xy && fits) {
+        // s = M u, + t, + c: the operations of avg_sample, two planes at a time.  (With the last plane of
+        // an odd count its pair repeats it.)
+        unsigned long long mz[3], ts[3];
+        const unsigned long long uu = pack2(u, u), vv = pack2(v, v), cc = pack2((float)c, (float)c);
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+          mz[i] = pack2(m[3 * i + 2], m[3 * i + 2]);
+          ts[i] = pack2(sh[i], sh[i]);
+        }
+#pragma unroll
+        for (int q = 0; q < Z; q += 2) {
+          if (q < nz) {
+            const unsigned long long ww = pack2((float)(bz + q - c), (float)(bz + min(q + 1, nz - 1) - c));
+            unsigned long long sp[3];
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {
+              const unsigned long long a0 = pack2(m[3 * i], m[3 * i]), a1 = pack2(m[3 * i + 1], m[3 * i + 1]);
+              sp[i] = fadd2(fadd2(ffma2(a0, uu, ffma2(a1, vv, fmul2(mz[i], ww))), ts[i]), cc);
+            }
+            const float2 val = unpack2(avg_sample_staged2(s_box, base, sp));
+            acc[q] += val.x;
+            acc[q + 1] += val.y;
+          }
         }
       }
-    } else if (in_xy) {
+      staged = fits;
+    }
+    if (in_xy && !staged) {
 #pragma unroll
-      for (int q = 0; q < kBrickZ; ++q)
+      for (int q = 0; q < Z; ++q)
         if (q < nz) acc[q] += avg_sample(src, n, m, u, v, (float)(bz + q - c), sh, c);
     }
   }
   double s1 = 0.0, s2 = 0.0, s3 = 0.0;
   if (in_xy) {
 #pragma unroll
-    for (int q = 0; q < kBrickZ; ++q) {
+    for (int q = 0; q < Z; ++q) {
       if (q >= nz) break;
       const long i = ((long)(bz + q) * n + y) * n + x;
       const float r = pr.nsym > 1 ? acc[q] / (float)pr.nsym : acc[q];
@@ -323,19 +330,24 @@ __global__ void __launch_bounds__(256, 3) k_avg_rotate(const float* __restrict__
 static emc_status launch_rotate(const float* vols, long vol_stride, const int* vol_index, int n, const float* mats,
                                 const AvgParticle* parts, int nb, int use_shift, const float* mask, float bin_thr,
                                 float* out, AvgStats* stats, cudaStream_t st) {
-  const long bxy = (n + kBrickXY - 1) / kBrickXY, bz = (n + kBrickZ - 1) / kBrickZ;
-  const dim3 grid((unsigned)(bxy * bxy * bz), nb);
-  auto go = [&](auto kern) -> emc_status {
-    EMC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kAvgBoxBytes));
-    kern<<<grid, 256, kAvgBoxBytes, st>>>(vols, vol_stride, vol_index, n, mats, parts, use_shift, mask, bin_thr, out,
-                                          stats);
+  const long bxy = (n + kBrickXY - 1) / kBrickXY;
+  auto ctas = [&](int z) { return bxy * bxy * ((n + z - 1) / z); };
+  auto go = [&](auto kern, int z, size_t smem) -> emc_status {
+    if (smem) EMC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    kern<<<dim3((unsigned)ctas(z), nb), 256, smem, st>>>(vols, vol_stride, vol_index, n, mats, parts, use_shift, mask,
+                                                         bin_thr, out, stats);
     EMC_LAUNCH_CHECK();
     return EMC_OK;
   };
   const uintptr_t base = (uintptr_t)vols;
-  if (n % 4 == 0 && base % 16 == 0) return go(k_avg_rotate<4>);
-  if (n % 2 == 0 && base % 8 == 0) return go(k_avg_rotate<2>);
-  return go(k_avg_rotate<1>);
+  const int v = n % 4 == 0 && base % 16 == 0 ? 4 : n % 2 == 0 && base % 8 == 0 ? 2 : 1;
+  // Up to three CTAs per four SMs, thin bricks without staging: Average.add of one 33^3 window, four operators,
+  // with a weight (45 CTAs each) 92 -> 78 us, eight of 17^3 (96) 98 -> 79; at 128 CTAs staging is the better
+  // one again (64^3: 90 against 99, eight of 32^3 91 against 104).
+  if (4 * ctas(kBrickZ) * nb <= 3L * device_sm_count()) return go(k_avg_rotate<0, kThinZ>, kThinZ, 0);
+  if (v == 4) return go(k_avg_rotate<4, kBrickZ>, kBrickZ, kAvgBoxBytes);
+  if (v == 2) return go(k_avg_rotate<2, kBrickZ>, kBrickZ, kAvgBoxBytes);
+  return go(k_avg_rotate<1, kBrickZ>, kBrickZ, kAvgBoxBytes);
 }
 
 // Copies a batch's parameters from the mapped host staging into device memory (the symmetry

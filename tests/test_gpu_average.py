@@ -131,11 +131,12 @@ def test_brick_edges_and_wide_matrices(built_lib, cuda, n, nw):
             assert np.abs(a - b).max() <= 2e-5 * np.abs(b).max(), (h, k)
 
 
-def test_cancelling_matrices_on_thin_bricks(built_lib, cuda):
+@pytest.mark.parametrize("windows", [1, 12])
+def test_cancelling_matrices_on_thin_bricks(built_lib, cuda, windows):
     """A box one voxel longer than whole bricks, with matrices whose entries are huge and cancel (or are
     cancelled by the shift) at its far corner: the sums in different orders differ by whole voxels there,
     so those samples do not come from the staged box.  The window's samples lie beyond it almost
-    everywhere; against a float32 restatement of the sampling in the kernel's order (FP32 products are
+    everywhere; with one window (too few CTAs to stage) and with several equal ones; against a float32 restatement of the sampling in the kernel's order (FP32 products are
     exact in float64, so one rounding each), whose coordinates must agree bit for bit."""
     from emclarity_b200 import api
     n, c = 17, 8
@@ -169,9 +170,32 @@ def test_cancelling_matrices_on_thin_bricks(built_lib, cuda):
                 idx.append(np.clip(b + oi, 0, n - 1).astype(int))
             want += np.where(ok, w * vol[idx[2], idx[1], idx[0]], 0.0)
         av = api.Average(mask)
-        kept = av.add(torch.from_numpy(vol)[None].cuda(), [m], [1], shifts=[t])
-        assert kept[0]
+        kept = av.add(torch.from_numpy(np.stack([vol] * windows)).cuda(), [m] * windows, [1] * windows,
+                      shifts=[t] * windows)
+        assert kept.all()
         got = av.result(1)[0].cpu().numpy()
         av.close()
         want = (want - want.mean()) / want.std()
         assert np.abs(got - want).max() <= 2e-5 * np.abs(want).max()
+
+
+@pytest.mark.parametrize("n,nw", [(17, 16), (33, 31), (40, 34)])
+def test_one_window_at_a_time_matches_a_batch(built_lib, cuda, n, nw):
+    """Few CTAs (one window) sample global memory in thin bricks, a batch stages boxes: the rotated values
+    are the same, the FP64 statistics differ by their order, so the sums differ by a rounding of each
+    window's mean, rms and quotient."""
+    c = _case(n, n=n, k=24, nw=nw)
+    from emclarity_b200 import api
+    sums = []
+    for step in (24, 1):
+        av = api.Average(torch.from_numpy(c["mask"]).cuda(), symmetry="C3", wedge_box=nw)
+        for i in range(0, 24, step):
+            j = slice(i, i + step)
+            kept = av.add(torch.from_numpy(c["parts"][j]).cuda(), c["rots"][j], c["halves"][j], shifts=c["shifts"][j],
+                          weights=c["weights"][j], wedges=torch.from_numpy(c["wedges"]).cuda(), wedge_index=c["widx"][j])
+            assert kept.all()
+        sums.append([[t.cpu().numpy() for t in av.result(h)[:2]] for h in (1, 2)])
+        av.close()
+    for a, b in zip(*sums):
+        assert np.abs(a[0] - b[0]).max() <= 4 * 12 * 2.0 ** -24 * np.abs(a[0]).max()
+        assert np.array_equal(a[1], b[1])
