@@ -491,8 +491,9 @@ bool mavg_tiled(int nx, int ny, int nz, int L) {
 
 // The three passes over a volume through a ring of xy-smoothed planes: slabs of z planes are
 // smoothed in x and y into the ring, then the outputs whose inputs are all there are formed along z.
-// The ring holds a slab and the L - 1 planes before it, sized to stay in the L2, so the smoothed
-// planes do not pass through HBM and the scratch does not grow with the volume.  vol may be `in`: a
+// The ring holds a slab of 64 MiB (at least kMavgZ planes) and the L - 1 planes before it: for tomograms of
+// 512 x 512 and features up to 29 it stays in the L2 (94 MiB at 16, 120 at 29), so that the smoothed planes
+// do not pass through HBM, and the scratch grows with a plane's area but not with nz.  vol may be `in`: a
 // slab's outputs end h planes below the planes that later slabs still read.
 template <bool SQ>
 emc_status mavg_ring(const float* in, float* vol, int nx, int ny, int nz, const std::vector<float>& w,

@@ -238,7 +238,7 @@ struct emc_search_s {
   emc::DevBuf<double> d_dmat;
   int norient = 0;
   int radius = 0, interp = EMC_INTERP_LINEAR, chunk_evals = 0;
-  // S1 + S2 scratch of a chunk: 768 MiB (about 545 evaluations at 64^3, 180 at 96^3, 80 at 128^3 with
+  // S1 + S2 scratch of a chunk: 768 MiB (546 evaluations at 64^3, 180 at 96^3, 80 at 128^3 with
   // radius 7), or an eighth of the free device memory if that is less.  Larger chunks amortise the
   // passes' launch tails, and the spectra that then spill from L2 cost HBM bandwidth the passes leave
   // unused: one slot at 64^3 takes 2,402 ns per evaluation at 32 evaluations per chunk, 1,783 at 256,

@@ -299,7 +299,7 @@ EMC_API emc_status emc_search_set_orientations(emc_search_t s, const double* phi
 /* Tuning knobs (0 = automatic / autotuned).  peak_radius: spherical peak mask radius in
  * voxels (the peakMask >= 0.95 region of BH_multi_xcf_Translational.m:34).  chunk_evals:
  * evaluations per launch of the three passes; 0 cuts each box's evaluations into equal chunks of
- * at most 768 MiB of scratch (about 520 evaluations at 64^3), or an eighth of the free device
+ * at most 768 MiB of scratch (546 evaluations at 64^3 and radius 7), or an eighth of the free device
  * memory at creation if less, and into at least two at 64^3 (whose chunks overlap in pairs). */
 EMC_API emc_status emc_search_configure(emc_search_t s, int peak_radius, int interp, int chunk_evals);
 /* Runs every (particle, orientation) pair.  d_cc / d_peak (optional, may be NULL):
@@ -455,11 +455,16 @@ EMC_API emc_status emc_tsearch_peaks(float* d_mag, const float* d_ang, int nx, i
                                      float high_thr, float sampling, double* h_peaks, int* n_found,
                                      void* stream);
 /* BH_movingAverage_2(img, featureSize) (statistics/BH_movingAverage_2.m): separable Gaussian
- * moving average (length featureSize, sigma 3, symmetric boundaries). */
+ * moving average (length featureSize, sigma 3, symmetric boundaries).  Runs in the order of `stream`:
+ * the call may return before it has finished, so another stream or the host waits for `stream`
+ * before it reads the result (features above 96 synchronise it).  Scratch from the stream-ordered
+ * allocator: min(nz, slab + featureSize - 1) planes of 4 bytes per voxel, a slab being the planes in
+ * 64 MiB and at least 32 (above 96: one volume). */
 EMC_API emc_status emc_moving_average(const float* d_in, int nx, int ny, int nz, int feature_size,
                                       float* d_out, void* stream);
 /* The local normalisation of BH_templateSearch3d_2.m:558-561, in place:
- * x <- (x - avg(x)) / sqrt(avg(x^2) - avg(x)^2) with avg = emc_moving_average. */
+ * x <- (x - avg(x)) / sqrt(avg(x^2) - avg(x)^2) with avg = emc_moving_average, in the order of
+ * `stream` as there; scratch planes of 8 bytes per voxel (above 96: four volumes). */
 EMC_API emc_status emc_local_normalize(float* d_vol, int nx, int ny, int nz, int feature_size, void* stream);
 
 /* ------------------------------------------------------------------------ */
