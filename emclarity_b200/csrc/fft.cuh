@@ -1,11 +1,14 @@
 // fft.cuh -- hand-written FP32 FFT building blocks for sm_100a.
 //
-// A line of length L (L = 2^a 3^b) is transformed in place in shared memory by a
-// "team" of P lanes of one warp (P divides 32).  Stages follow the Stockham
-// autosort formulation with mixed radices {2,3,4,8,16}: each lane loads all the
-// inputs of its butterflies into registers, the warp synchronises, then the lane
-// applies twiddles, runs the radix-R DFT codelet in registers and stores.  With
-// two or three stages per line, data crosses shared memory 2-3 times per axis.
+// Register codelets of radix 2, 3, 4, 5, 7, 8, 12, 13 and 16, in two forms of a mixed-radix transform:
+//
+// * teams (fft_line, Stockham stages): a line in shared memory is transformed by P lanes of one warp (P
+//   divides 32).  Each lane loads all the inputs of its butterflies into registers, the warp
+//   synchronises, then the lane applies twiddles, runs the codelet and stores.  For contiguous lines: the
+//   rows of the standalone transform and of the template search, the search's pass C.
+// * lines across lanes (InPlace): neighbouring threads hold neighbouring lines and one butterfly each,
+//   stages work in place, and only the exchanges between stages cross shared memory.  For strided axes:
+//   k_cols, the template search's z pass; the search's passes A and B have their own two-stage variant.
 //
 // Sign convention: SIGN = -1 is the forward transform X_k = sum x_n e^{-2 pi i nk/L}
 // (cuFFT / MATLAB fftn), SIGN = +1 the unnormalised inverse.
@@ -302,13 +305,6 @@ __host__ __device__ constexpr int radix_of(int L, int s) {
 __host__ __device__ constexpr int max_radix(int L, int s = 0) {
   return radix_of(L, s) <= 1 ? 1
          : (radix_of(L, s) > max_radix(L, s + 1) ? radix_of(L, s) : max_radix(L, s + 1));
-}
-// Complex values a lane of a P-lane team holds in the largest stage of a length-L line.
-__host__ __device__ constexpr int stage_values(int L, int P, int s = 0) {
-  return radix_of(L, s) <= 1 ? 0
-         : ((L / radix_of(L, s) + P - 1) / P) * radix_of(L, s) > stage_values(L, P, s + 1)
-             ? ((L / radix_of(L, s) + P - 1) / P) * radix_of(L, s)
-             : stage_values(L, P, s + 1);
 }
 __host__ __device__ constexpr int min_butterflies(int L) { return radix_of(L, 0) == 0 ? 0 : L / max_radix(L); }
 
